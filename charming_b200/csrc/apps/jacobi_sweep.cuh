@@ -170,6 +170,58 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, unsigned 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
+// The multi-sweep pass's ring of rows, addressed in the shared window, and
+// its stores: the first n of a lane's VEC values (n >= VEC: one 16-byte
+// store), predicated so that the row loop has no branch in it.
+using ring_addr = unsigned;
+__device__ __forceinline__ ring_addr to_ring(void* p) { return smem_u32(p); }
+__device__ __forceinline__ void ring_fetch(ring_addr a, const void* src, unsigned src_bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(a), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ void ring_read(ring_addr a, double (&x)[2]) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x[0]), "=d"(x[1]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ring_read(ring_addr a, float (&x)[4]) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void put_vec(double* p, const double (&x)[2], int n) {
+  asm volatile("{\n .reg .pred f, h;\n setp.ge.s32 f, %3, 2;\n setp.eq.s32 h, %3, 1;\n"
+               " @f st.global.v2.f64 [%0], {%1, %2};\n @h st.global.f64 [%0], %1;\n}"
+               :: "l"(p), "d"(x[0]), "d"(x[1]), "r"(n) : "memory");
+}
+__device__ __forceinline__ void put_vec(float* p, const float (&x)[4], int n) {
+  asm volatile("{\n .reg .pred f, a, b, c;\n setp.ge.s32 f, %5, 4;\n setp.eq.s32 a, %5, 1;\n"
+               " setp.eq.s32 c, %5, 3;\n setp.eq.or.s32 b, %5, 2, c;\n"
+               " @f st.global.v4.f32 [%0], {%1, %2, %3, %4};\n @b st.global.v2.f32 [%0], {%1, %2};\n"
+               " @a st.global.f32 [%0], %1;\n @c st.global.f32 [%0+8], %3;\n}"
+               :: "l"(p), "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]), "r"(n) : "memory");
+}
+// Two floats in one instruction, each with the rounding of the single one.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
 __device__ __forceinline__ bool mbar_test_wait(unsigned long long* b, unsigned parity) {
   unsigned done;
   asm volatile(
@@ -197,6 +249,19 @@ inline void cp_async16(void* dst, const void* src, unsigned src_bytes) {
 }
 inline void cp_async_commit() {}
 template <int N> inline void cp_async_wait() {}
+using ring_addr = char*;
+inline ring_addr to_ring(void* p) { return static_cast<char*>(p); }
+inline void ring_fetch(ring_addr a, const void* src, unsigned src_bytes) { cp_async16(a, src, src_bytes); }
+template <typename T, int V> inline void ring_read(ring_addr a, T (&x)[V]) { memcpy(x, a, 16); }
+template <typename T, int V> inline void put_vec(T* p, const T (&x)[V], int n) {
+  for (int k = 0; k < V && k < n; k++) p[k] = x[k];
+}
+struct f32x2 { float a, b; };
+inline f32x2 pack2(float a, float b) { return {a, b}; }
+inline void unpack2(f32x2 v, float& a, float& b) { a = v.a; b = v.b; }
+inline f32x2 add2(f32x2 x, f32x2 y) { return {x.a + y.a, x.b + y.b}; }
+inline f32x2 mul2(f32x2 x, f32x2 y) { return {x.a * y.a, x.b * y.b}; }
+inline f32x2 fma2(f32x2 x, f32x2 y, f32x2 z) { return {fmaf(x.a, y.a, z.a), fmaf(x.b, y.b, z.b)}; }
 #endif
 
 // ---------------------------------------------------------------------------
@@ -382,15 +447,15 @@ __device__ __noinline__ double sweep_direct(block_view<T> in, block_view<T> out,
 // grid whose ghost zone is at least L deep, without writing the
 // intermediate sweeps. A warp owns a strip of 32 vectors (one per lane) and
 // streams level-0 rows down it; level l row r is computed when level l-1
-// row r+1 arrives, from a three-row register window per level, so the pass
-// is a wavefront L rows deep. Every level loses one valid column at each
-// strip edge (the neighbour value is in another warp), so strips overlap by
-// 2*ceil(L/VEC) vectors and each owns the 32 - 2*ceil(L/VEC) in the middle;
-// row runs overlap by 2L rows. Cells on the domain boundary (row 0 / h+1,
-// column 0 / w+1 of a chare without a neighbour there) keep their value at
-// every level; cells beyond it are never used by a stored result. Each
-// stored value is computed from the same five operands in the same order as
-// a single sweep, so L passes of one sweep give the same bits.
+// row r+1 arrives, so the pass is a wavefront L rows deep. Every level loses
+// one valid column at each strip edge (the neighbour value is in another
+// warp), so strips overlap by 2*ceil(L/VEC) vectors and each owns the
+// 32 - 2*ceil(L/VEC) in the middle; row runs overlap by 2L rows. Cells on
+// the domain boundary (row 0 / h+1, column 0 / w+1 of a chare without a
+// neighbour there) keep their value at every level; cells beyond it are
+// never used by a stored result. Each stored value is computed from the
+// same five operands in the same order as a single sweep, so L passes of
+// one sweep give the same bits.
 // `fixed`: bit 0 top, 1 bottom, 2 left, 3 right side is the domain boundary.
 // ---------------------------------------------------------------------------
 template <typename T>
@@ -436,181 +501,181 @@ __device__ __forceinline__ deep_lane<T> make_lane(int w, int h, int fixed, int o
   return ln;
 }
 
-// All L levels of the wavefront at sub-step K of a three-step cycle (level-l
-// row r lives in W[l][(r - qs) mod 3], so every window index is static).
-// CHECK: a level runs only once its three input rows exist (the first 2L
-// steps of an item). Domain-boundary cells keep their value at every level:
-// a whole row by a warp-uniform branch, a column by a per-lane fix-up.
-// ROWFIX / COLFIX false: the step cannot meet a domain-boundary row / the
-// strip holds no domain-boundary column, so those tests are left out.
-template <typename T, bool RESID, int L, int K, bool CHECK, bool ROWFIX = true, bool COLFIX = true>
-__device__ __forceinline__ void deep_step(typename vec_of<T>::type (&W)[L][3], int q, int qs, int w,
-    const deep_lane<T>& ln, int r0, int r1, const block_view<T>& out, double& acc) {
+// What a lane keeps per level between two rows: the newest row of the level
+// below (X) and the partial sums ((c + l) + r) + u around it (P), taken as
+// soon as that row arrived. When the next row d arrives, the level's output
+// is (P + d) * 0.2: the same adds in the same order as `stencil`, but one
+// add and one multiply (not two shuffles and five operations) lie between
+// the rows of two levels, so a step's chain through the L levels is 2L
+// operations long, and two rows per level (three when the whole window is
+// kept) fit in registers.
+template <typename T, int L>
+struct deep_state {
+  T P[L][traits<T>::VEC], X[L][traits<T>::VEC];
+  double D[traits<T>::VEC];  // level 1's partial sums in FP64 (residual of float grids)
+};
+
+__device__ __forceinline__ double resid_close(double p, double d) { return __dmul_rn(__dadd_rn(p, d), 0.2); }
+// (P + x) * 0.2, rounded as `stencil` rounds it.
+__device__ __forceinline__ void close_vec(double (&o)[2], const double (&P)[2], const double (&x)[2]) {
+#pragma unroll
+  for (int k = 0; k < 2; k++) o[k] = resid_close(P[k], x[k]);
+}
+__device__ __forceinline__ void close_vec(float (&o)[4], const float (&P)[4], const float (&x)[4]) {
+  const f32x2 hi = pack2(STENCIL_C_HI, STENCIL_C_HI), lo = pack2(STENCIL_C_LO, STENCIL_C_LO);
+#pragma unroll
+  for (int k = 0; k < 4; k += 2) {
+    const f32x2 s = add2(pack2(P[k], P[k + 1]), pack2(x[k], x[k + 1]));
+    unpack2(fma2(s, hi, mul2(s, lo)), o[k], o[k + 1]);
+  }
+}
+// P = ((x + l) + r) + X.
+__device__ __forceinline__ void open_vec(double (&P)[2], const double (&x)[2], const double (&X)[2], double left,
+    double right) {
+  P[0] = __dadd_rn(__dadd_rn(__dadd_rn(x[0], left), x[1]), X[0]);
+  P[1] = __dadd_rn(__dadd_rn(__dadd_rn(x[1], x[0]), right), X[1]);
+}
+__device__ __forceinline__ void open_vec(float (&P)[4], const float (&x)[4], const float (&X)[4], float left,
+    float right) {
+  float t[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    t[k] = __fadd_rn(__fadd_rn(x[k], k == 0 ? left : x[k - 1]), k == 3 ? right : x[k + 1]);
+#pragma unroll
+  for (int k = 0; k < 4; k += 2)
+    unpack2(add2(pack2(t[k], t[k + 1]), pack2(X[k], X[k + 1])), P[k], P[k + 1]);
+}
+
+// One step of the wavefront through levels 1..LM: level-0 row q arrives in x,
+// level l's row q - l is computed; x leaves as the row of level LM. FIX: the
+// domain boundary is looked for (its cells keep their value at every level);
+// without it the step must not meet one. There is no branch in a step: a
+// branch in the row loop cost two register moves per value and level.
+template <typename T, bool RESID, int L, int LM, bool FIX>
+__device__ __forceinline__ void deep_step(deep_state<T, L>& S, T (&x)[traits<T>::VEC], int q,
+    const deep_lane<T>& ln, int r0, int r1, double& acc) {
   constexpr int V = traits<T>::VEC;
   constexpr unsigned FULL = 0xffffffffu;
-  using VT = typename vec_of<T>::type;
 #pragma unroll
-  for (int l = 1; l <= L; l++) {
-    if (CHECK && q < qs + 2 * l) continue;
-    const int r = q - l;  // row of level l computed now
-    const int su = ((K - l - 1) % 3 + 6) % 3, sm = ((K - l) % 3 + 6) % 3, sd = ((K - l + 1) % 3 + 6) % 3;
-    T m[V], u[V], d[V], o[V];
-    vec_to<T>(W[l - 1][sm], m);
-    vec_to<T>(W[l - 1][su], u);
-    vec_to<T>(W[l - 1][sd], d);
-    T left = __shfl_up_sync(FULL, m[V - 1], 1);
-    T right = __shfl_down_sync(FULL, m[0], 1);
-    if (ROWFIX && (r == ln.fix_r0 || r == ln.fix_r1)) {  // domain-boundary row: kept (warp-uniform)
-#pragma unroll
-      for (int k = 0; k < V; k++) o[k] = m[k];
-    } else {
+  for (int l = 1; l <= LM; l++) {
+    const T left = __shfl_up_sync(FULL, x[V - 1], 1);
+    const T right = __shfl_down_sync(FULL, x[0], 1);
+    T o[V];
+    close_vec(o, S.P[l - 1], x);
+    if (RESID && l == 1) {
 #pragma unroll
       for (int k = 0; k < V; k++) {
-        T lk = (k == 0) ? left : m[k - 1];
-        T rk = (k == V - 1) ? right : m[k + 1];
-        o[k] = stencil(m[k], lk, rk, u[k], d[k]);
-        if (RESID && l == 1 && ln.own && ln.inw[k] && r >= r0 && r < r1)
-          acc += resid2<T>(m[k], lk, rk, u[k], d[k]);
-      }
-      if (COLFIX && ln.anyfix) {  // the lane holding column 0 or w+1 of the domain
-#pragma unroll
-        for (int k = 0; k < V; k++)
-          if (ln.fixc[k]) o[k] = m[k];
-      }
-    }
-    if (l == L) {
-      if (ln.own) {
-        T* op = out.at(r, ln.col0);
-        int nvalid = w - ln.v * V;
-        if (nvalid >= V) {
-          *reinterpret_cast<VT*>(op) = vec_from(o);
-        } else {
-          #pragma unroll
-        for (int k = 0; k < V; k++)  // static indices keep o[] in registers
-          if (k < nvalid) op[k] = o[k];
+        const double c = (double)S.X[0][k];
+        const double s = sizeof(T) == 8 ? (double)o[k] : resid_close(S.D[k], (double)x[k]);
+        const double e = __dsub_rn(s, c);
+        if (ln.own && ln.inw[k] && q - 1 >= r0 && q - 1 < r1) acc += __dmul_rn(e, e);
+        if (sizeof(T) == 4) {
+          const double lk = (double)(k == 0 ? left : x[k - 1]), rk = (double)(k == V - 1 ? right : x[k + 1]);
+          S.D[k] = __dadd_rn(__dadd_rn(__dadd_rn((double)x[k], lk), rk), c);
         }
       }
-    } else {
-      W[l][sm] = vec_from(o);
+    }
+    if (FIX) {
+      const bool row = q - l == ln.fix_r0 || q - l == ln.fix_r1;
+#pragma unroll
+      for (int k = 0; k < V; k++) o[k] = (row || ln.fixc[k]) ? S.X[l - 1][k] : o[k];
+    }
+    open_vec(S.P[l - 1], x, S.X[l - 1], left, right);
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      S.X[l - 1][k] = x[k];
+      x[k] = o[k];
     }
   }
 }
 
-// One strip item: level-0 rows stream through this lane's private ring of P
-// 16-byte slots in shared memory (cp.async, P-1 rows ahead), the levels
-// through registers.
+// The level-0 rows of one lane, in order, through its private ring of P
+// 16-byte slots in shared memory (cp.async, P-1 rows ahead; slots lie 32
+// vectors apart), so no barrier is needed around it.
 template <typename T, int P>
-__device__ __forceinline__ void deep_fetch(typename vec_of<T>::type* ring, int lane, int& slot, int q,
-    int qe, const block_view<T>& in, long long eo, unsigned nb, typename vec_of<T>::type& x) {
-  cp_async_wait<P - 2>();
-  x = ring[slot * 32 + lane];
-  const int nslot = slot == 0 ? P - 1 : slot - 1;  // slot of row q-1, read last step
-  if (q + P - 1 <= qe) cp_async16(&ring[nslot * 32 + lane], in.row(q + P - 1) + eo, nb);
-  cp_async_commit();
-  slot = slot + 1 == P ? 0 : slot + 1;
-}
+struct deep_stream {
+  ring_addr ring;  // this lane's slot 0
+  const T* next;   // this lane's vector of the next row to fetch
+  int left;        // rows not yet fetched
+  int pitch;
+  unsigned at;     // byte offset of the next row's slot
+  unsigned nb;     // 16, or 0 (zero fill) for a vector outside the pitched row
+  __device__ __forceinline__ void fetch(unsigned slot) {
+    ring_fetch(ring + slot, next, nb);
+    cp_async_commit();
+    left--;
+    next += left > 0 ? pitch : 0;  // after the last row: that row again, never used
+  }
+  __device__ __forceinline__ void pop(T (&x)[traits<T>::VEC]) {
+    cp_async_wait<P - 2>();
+    ring_read(ring + at, x);
+    fetch((at + (P - 1) * 512) & (P * 512 - 1));  // the slot of the row read before
+    at = (at + 512) & (P * 512 - 1);
+  }
+};
 
+// One strip item, in four loops: the first half of the fill (L steps, in
+// which only the lower half of the levels has a row to work on), the second
+// half, the steady steps, and the steps at the bottom domain boundary.
+// Level l computes row q - l, so its first row is complete at step qs + 2l,
+// and levels 1..L-1 meet the bottom boundary row R at steps R+1..R+L-1. The
+// steady loop has no boundary tests (it takes no strip that holds a
+// domain-boundary column); it takes 4 rows per turn, so that the rows a lane
+// keeps need few register moves. sweep alone, 148 blocks of 2048 x 221, FP64, 6 levels:
+// 272 us per pass (1480 GLUP/s), 327 with the whole window kept and a branch
+// per level; FP32 155 us (199); 128 x 128 FP64 25.8 us (31.9). The FP64
+// pipe is 55 % busy, the shuffles' pipe 58 %, the issue slots 74 %.
 template <typename T, bool RESID, int L, int P>
 __device__ __forceinline__ double deep_item(const block_view<T>& in, const block_view<T>& out, int w,
-    const deep_lane<T>& ln, int r0, int r1, int lane, typename vec_of<T>::type* ring) {
-  constexpr int V = traits<T>::VEC;
-  using VT = typename vec_of<T>::type;
+    const deep_lane<T>& ln, int r0, int r1, int lane, typename vec_of<T>::type* ring, bool lean) {
+  constexpr int V = traits<T>::VEC, LH = (L + 1) / 2, U = 4;
   const long long e0 = (long long)traits<T>::OFF - 1 + ln.col0;  // element index in a row
   const bool can_load = e0 >= 0 && e0 + V <= in.pitch;
-  const long long eo = can_load ? e0 : 0;
-  const unsigned nb = can_load ? 16u : 0u;
-  const int qs = r0 - L, qe = r1 - 1 + L;             // level-0 rows streamed
-#pragma unroll
-  for (int k = 0; k < P - 1; k++) {
-    if (qs + k <= qe) cp_async16(&ring[k * 32 + lane], in.row(qs + k) + eo, nb);
-    cp_async_commit();
-  }
-  VT W[L][3];
-  double acc = 0.0;
-  int slot = 0;                                       // ring slot of row q
-  // fill: until every level has its three rows (checked steps)
-  constexpr int F = (2 * L + 2) / 3 * 3;
-  int q0 = qs;
-  for (; q0 < qs + F && q0 <= qe; q0 += 3) {
-#pragma unroll
-    for (int K = 0; K < 3; K++) {
-      const int q = q0 + K;
-      if (q > qe) break;
-      deep_fetch<T, P>(ring, lane, slot, q, qe, in, eo, nb, W[0][K]);
-      if (K == 0) deep_step<T, RESID, L, 0, true>(W, q, qs, w, ln, r0, r1, out, acc);
-      else if (K == 1) deep_step<T, RESID, L, 1, true>(W, q, qs, w, ln, r0, r1, out, acc);
-      else deep_step<T, RESID, L, 2, true>(W, q, qs, w, ln, r0, r1, out, acc);
-    }
-  }
-  // steady state: all levels every step
-  for (; q0 <= qe; q0 += 3) {
-#pragma unroll
-    for (int K = 0; K < 3; K++) {
-      const int q = q0 + K;
-      if (q > qe) break;
-      deep_fetch<T, P>(ring, lane, slot, q, qe, in, eo, nb, W[0][K]);
-      if (K == 0) deep_step<T, RESID, L, 0, false>(W, q, qs, w, ln, r0, r1, out, acc);
-      else if (K == 1) deep_step<T, RESID, L, 1, false>(W, q, qs, w, ln, r0, r1, out, acc);
-      else deep_step<T, RESID, L, 2, false>(W, q, qs, w, ln, r0, r1, out, acc);
-    }
-  }
-  cp_async_wait<0>();
-  return acc;
-}
-
-// ---------------------------------------------------------------------------
-// The same item, with the tests taken out of the steady state: a group of
-// three steps that cannot need them (past the fill, before the steps that
-// can meet the bottom boundary row, in a strip without a domain-boundary
-// column) runs a step without the fill check, the boundary-row test and the
-// column fix-up; the other groups run the general step. One loop and two
-// step versions keep the code (and so the instruction cache footprint) as
-// small as deep_item's. Same arithmetic and results as deep_item.
-// ---------------------------------------------------------------------------
-template <typename T, bool RESID, int L, int P>
-__device__ __forceinline__ double lean_item(const block_view<T>& in, const block_view<T>& out, int w,
-    const deep_lane<T>& ln, int r0, int r1, int lane, typename vec_of<T>::type* ring) {
-  constexpr int V = traits<T>::VEC;
-  using VT = typename vec_of<T>::type;
-  const long long e0 = (long long)traits<T>::OFF - 1 + ln.col0;  // element index in a row
-  const bool can_load = e0 >= 0 && e0 + V <= in.pitch;
-  const long long eo = can_load ? e0 : 0;
-  const unsigned nb = can_load ? 16u : 0u;
   const int qs = r0 - L, qe = r1 - 1 + L;  // level-0 rows streamed
-  constexpr int F = (2 * L + 2) / 3 * 3;   // steps of the fill (every level has its rows after)
-  // steady groups: from the end of the fill to before the first step at
-  // which a level can compute the bottom boundary row R (level l computes
-  // row q - l, so levels 1..L-1 reach R at steps R+1..R+L-1); none in a
-  // strip holding a domain-boundary column
   int q_lean_end = (ln.fix_r1 != INT_MIN && ln.fix_r1 + 1 <= qe) ? ln.fix_r1 + 1 : qe + 1;
-  if (__any_sync(0xffffffffu, ln.anyfix)) q_lean_end = INT_MIN;
+  if (!lean || __any_sync(0xffffffffu, ln.anyfix)) q_lean_end = INT_MIN;
+  deep_stream<T, P> st{to_ring(ring + lane), in.row(qs) + (can_load ? e0 : 0), qe - qs + 1, in.pitch, 0,
+                       can_load ? 16u : 0u};
 #pragma unroll
-  for (int k = 0; k < P - 1; k++) {
-    if (qs + k <= qe) cp_async16(&ring[k * 32 + lane], in.row(qs + k) + eo, nb);
-    cp_async_commit();
-  }
-  VT W[L][3];
+  for (int k = 0; k < P - 1; k++) st.fetch(k * 512);
+  deep_state<T, L> S;
+#pragma unroll
+  for (int l = 0; l < L; l++)
+#pragma unroll
+    for (int k = 0; k < V; k++) S.P[l][k] = S.X[l][k] = (T)0;
+#pragma unroll
+  for (int k = 0; k < V; k++) S.D[k] = 0.0;
   double acc = 0.0;
-  int slot = 0;
-  for (int q0 = qs; q0 <= qe; q0 += 3) {
-    if (q0 >= qs + F && q0 + 2 < q_lean_end) {
-      deep_fetch<T, P>(ring, lane, slot, q0, qe, in, eo, nb, W[0][0]);
-      deep_step<T, RESID, L, 0, false, false, false>(W, q0, qs, w, ln, r0, r1, out, acc);
-      deep_fetch<T, P>(ring, lane, slot, q0 + 1, qe, in, eo, nb, W[0][1]);
-      deep_step<T, RESID, L, 1, false, false, false>(W, q0 + 1, qs, w, ln, r0, r1, out, acc);
-      deep_fetch<T, P>(ring, lane, slot, q0 + 2, qe, in, eo, nb, W[0][2]);
-      deep_step<T, RESID, L, 2, false, false, false>(W, q0 + 2, qs, w, ln, r0, r1, out, acc);
-    } else {
+  T x[V];
+  T* op = out.row(r0) + e0;
+  const int nput = ln.own ? w - ln.v * V : 0;
+  int q = qs;
+#pragma unroll 1
+  for (; q < qs + 2 * LH; q++) {
+    st.pop(x);
+    deep_step<T, RESID, L, LH, true>(S, x, q, ln, r0, r1, acc);
+  }
+#pragma unroll 1
+  for (; q < qs + 2 * L; q++) {
+    st.pop(x);
+    deep_step<T, RESID, L, L, true>(S, x, q, ln, r0, r1, acc);
+  }
+#pragma unroll 1
+  for (; q + U - 1 < q_lean_end; q += U) {
 #pragma unroll
-      for (int K = 0; K < 3; K++) {
-        const int q = q0 + K;
-        if (q > qe) break;
-        deep_fetch<T, P>(ring, lane, slot, q, qe, in, eo, nb, W[0][K]);
-        if (K == 0) deep_step<T, RESID, L, 0, true>(W, q, qs, w, ln, r0, r1, out, acc);
-        else if (K == 1) deep_step<T, RESID, L, 1, true>(W, q, qs, w, ln, r0, r1, out, acc);
-        else deep_step<T, RESID, L, 2, true>(W, q, qs, w, ln, r0, r1, out, acc);
-      }
+    for (int u = 0; u < U; u++) {
+      st.pop(x);
+      deep_step<T, RESID, L, L, false>(S, x, q + u, ln, r0, r1, acc);
+      put_vec(op, x, nput);
+      op += out.pitch;
     }
+  }
+#pragma unroll 1
+  for (; q <= qe; q++) {
+    st.pop(x);
+    deep_step<T, RESID, L, L, true>(S, x, q, ln, r0, r1, acc);
+    put_vec(op, x, nput);
+    op += out.pitch;
   }
   cp_async_wait<0>();
   return acc;
@@ -659,9 +724,9 @@ __device__ double sweep_deep_simple(block_view<T> in, block_view<T> out, int w, 
 }
 
 // The items of one pass of L sweeps (one warp); one register allocation per L.
-template <typename T, bool RESID, int L, bool LEAN>
+template <typename T, bool RESID, int L>
 __device__ __noinline__ double sweep_deep_items(block_view<T> in, block_view<T> out, int w, int h,
-    int fixed, typename vec_of<T>::type* ring, int nw, int warp, int lane) {
+    int fixed, typename vec_of<T>::type* ring, int nw, int warp, int lane, bool lean) {
   constexpr int V = traits<T>::VEC, P = 8;
   constexpr int E = (L + V - 1) / V;    // vectors lost at each strip edge over L levels
   constexpr int SS = 32 - 2 * E;        // vectors a strip owns
@@ -686,14 +751,13 @@ __device__ __noinline__ double sweep_deep_items(block_view<T> in, block_view<T> 
     int own0 = s * SS;
     int nown = min(SS, nv - own0);
     const deep_lane<T> ln = make_lane<T, L>(w, h, fixed, own0, nown, lane);
-    if (LEAN) acc += lean_item<T, RESID, L, P>(in, out, w, ln, r0, r1, lane, ring);
-    else acc += deep_item<T, RESID, L, P>(in, out, w, ln, r0, r1, lane, ring);
+    acc += deep_item<T, RESID, L, P>(in, out, w, ln, r0, r1, lane, ring, lean);
   }
   return acc;
 }
 
-// lean: the phase-split items (lean_item) instead of deep_item; same
-// results bit for bit.
+// lean: steps that need no boundary or fill tests leave them out (false:
+// every step tests); same results bit for bit.
 template <typename T, bool RESID>
 __device__ __noinline__ double sweep_deep(block_view<T> in, block_view<T> out, int w, int h, int L,
     int fixed, bool lean = true) {
@@ -710,9 +774,7 @@ __device__ __noinline__ double sweep_deep(block_view<T> in, block_view<T> out, i
   }
   VT* ring = rings + (size_t)warp * P * 32;
 #define CHARMING_DEEP_CASE(LL)                                                                 \
-  if (L == LL)                                                                                 \
-    return lean ? sweep_deep_items<T, RESID, LL, true>(in, out, w, h, fixed, ring, nw, warp, lane) \
-                : sweep_deep_items<T, RESID, LL, false>(in, out, w, h, fixed, ring, nw, warp, lane);
+  if (L == LL) return sweep_deep_items<T, RESID, LL>(in, out, w, h, fixed, ring, nw, warp, lane, lean);
   CHARMING_DEEP_CASE(2)
   CHARMING_DEEP_CASE(3)
   CHARMING_DEEP_CASE(5)
@@ -720,8 +782,7 @@ __device__ __noinline__ double sweep_deep(block_view<T> in, block_view<T> out, i
   CHARMING_DEEP_CASE(7)
   CHARMING_DEEP_CASE(8)
 #undef CHARMING_DEEP_CASE
-  return lean ? sweep_deep_items<T, RESID, 4, true>(in, out, w, h, fixed, ring, nw, warp, lane)
-              : sweep_deep_items<T, RESID, 4, false>(in, out, w, h, fixed, ring, nw, warp, lane);
+  return sweep_deep_items<T, RESID, 4>(in, out, w, h, fixed, ring, nw, warp, lane, lean);
 }
 
 // ---------------------------------------------------------------------------

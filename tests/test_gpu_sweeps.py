@@ -1,0 +1,48 @@
+"""GPU parity tests of the sweep kernels at the edges of their tiles and
+remainders (bit-exact against the CPU oracle; the arithmetic is the same
+operations in the same order, so there is no tolerance)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from charming_b200.jacobi import Jacobi2D, Problem
+from oracle import jacobi as oj
+
+pytestmark = pytest.mark.gpu
+
+
+def oracle(grid, sweeps):
+    if grid.dtype == np.float64:
+        return oj.jacobi2d(grid, sweeps)
+    g = np.ascontiguousarray(grid).copy()
+    oj.lib().oracle_jacobi2d_f32(g.ctypes.data_as(C.POINTER(C.c_float)), g.shape[1] - 2, g.shape[0] - 2, sweeps, 0)
+    return g
+
+
+def same_bits(a, b):
+    return np.array_equal(a.view(np.uint8), b.view(np.uint8))
+
+
+# widths around whole vectors (2 or 4 values) and strips (a warp owns 32 less
+# the vectors its edges lose), heights around the steady loop's turns of 4
+# rows after the fill of 2 * depth rows, one chare and split ones
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("depth", [2, 5, 6, 8])
+def test_multi_sweep_pass_tile_edges(rt, dtype, depth):
+    rng = np.random.default_rng(depth)
+    npdt = np.float64 if dtype == "f64" else np.float32
+    sizes = [(w, h) for w in (9, 48, 53, 104, 111, 117) for h in (8, 4 * depth + 1, 4 * depth + 2, 4 * depth + 3, 131)]
+    probs, grids = [], []
+    for k, (w, h) in enumerate(sizes):
+        px, py = ((1, 1), (1, 1), (2, 1), (1, 2), (2, 3))[k % 5]
+        if w // px < depth or h // py < depth:
+            px = py = 1
+        probs.append(Problem(w, h, 2 * depth + 3, px=px, py=py))
+        grids.append(rng.random((h + 2, w + 2)).astype(npdt))
+    with Jacobi2D(probs, dtype=dtype, depth=depth) as j:
+        for p, g in enumerate(grids):
+            j.load(p, g)
+        j.run()
+        for p, g in enumerate(grids):
+            assert same_bits(j.store(p), oracle(g, probs[p].max_sweeps)), sizes[p]
