@@ -32,6 +32,7 @@ struct JHandle {
   int* d_final = nullptr;
   int* d_block_map = nullptr;
   int* d_chare_of = nullptr;
+  double* d_bc = nullptr;                  // boundary values, 4 per problem
   unsigned long long* d_sweep_ns = nullptr;
   char* d_grid = nullptr;
   size_t grid_bytes = 0;
@@ -185,6 +186,11 @@ extern "C" int charming_jacobi2d_create(const charming_jacobi_problem* probs, in
   if (e == cudaSuccess) e = cudaMalloc(&h->d_block_map, sizeof(int) * n_pes);
   if (e == cudaSuccess) e = cudaMalloc(&h->d_chare_of, sizeof(int) * h->chare_of.size());
   if (e == cudaSuccess) e = cudaMalloc(&h->d_sweep_ns, 64 * (size_t)n_pes);
+  std::vector<double> bc(4 * (size_t)n);
+  for (int p = 0; p < n; p++)
+    for (int k = 0; k < 4; k++) bc[4 * (size_t)p + k] = probs[p].bc[k];
+  if (e == cudaSuccess) e = cudaMalloc(&h->d_bc, sizeof(double) * bc.size());
+  if (e == cudaSuccess) e = cudaMemcpy(h->d_bc, bc.data(), sizeof(double) * bc.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(h->d_chares, h->chares.data(), sizeof(jac::chare_desc) * nch, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(h->d_probs, pd.data(), sizeof(jac::prob_desc) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(h->d_results, 0, sizeof(jac::prob_result) * n);
@@ -194,6 +200,14 @@ extern "C" int charming_jacobi2d_create(const charming_jacobi_problem* probs, in
   if (e == cudaSuccess) e = cudaHostAlloc(&h->h_params, sizeof(suite::app_params), cudaHostAllocDefault);
   if (e == cudaSuccess) e = cudaEventCreate(&h->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&h->ev1);
+  if (e != cudaSuccess) {
+    rc = charm_host::cuda_fail(e, "jacobi2d descriptors");
+    charming_jacobi2d_destroy(h);
+    return rc;
+  }
+  // the copies and the zero fill above ran on the default stream, which the
+  // runtime's stream does not wait for
+  e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     rc = charm_host::cuda_fail(e, "jacobi2d descriptors");
     charming_jacobi2d_destroy(h);
@@ -225,21 +239,12 @@ extern "C" int charming_jacobi2d_create(const charming_jacobi_problem* probs, in
 extern "C" int charming_jacobi2d_init(void* handle) {
   JHandle* h = reinterpret_cast<JHandle*>(handle);
   if (!h) return CHARMING_ERR_CONFIG;
-  int n = (int)h->probs.size();
-  std::vector<double> bc(4 * n);
-  for (int p = 0; p < n; p++)
-    for (int k = 0; k < 4; k++) bc[4 * p + k] = h->probs[p].bc[k];
-  double* d_bc = nullptr;
-  cudaError_t e = cudaMalloc(&d_bc, sizeof(double) * bc.size());
-  if (e == cudaSuccess) e = cudaMemcpy(d_bc, bc.data(), sizeof(double) * bc.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) {
-    if (h->esz == 8) init_kernel<double><<<h->n_chares, 256>>>(h->d_chares, h->d_probs, d_bc);
-    else init_kernel<float><<<h->n_chares, 256>>>(h->d_chares, h->d_probs, d_bc);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
-  cudaFree(d_bc);
-  if (e == cudaSuccess) e = cudaMemset(h->d_final, 0, sizeof(int) * h->n_chares);
+  cudaStream_t s = charm_host::stream();
+  if (h->esz == 8) init_kernel<double><<<h->n_chares, 256, 0, s>>>(h->d_chares, h->d_probs, h->d_bc);
+  else init_kernel<float><<<h->n_chares, 256, 0, s>>>(h->d_chares, h->d_probs, h->d_bc);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->d_final, 0, sizeof(int) * h->n_chares, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   return check_cuda(e, "jacobi2d init");
 }
 
@@ -513,10 +518,10 @@ extern "C" int charming_jacobi2d_get_info(void* handle, charming_jacobi_info* ou
   // the per-PE phase timers count SM cycles
   std::vector<unsigned long long> ns(8 * h->block_map.size());
   cudaError_t e = cudaMemcpy(ns.data(), h->d_sweep_ns, 8 * ns.size(), cudaMemcpyDeviceToHost);
-  int dev = 0, khz = 0;
-  if (e == cudaSuccess) e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, dev);
   if (e != cudaSuccess) return check_cuda(e, "jacobi2d info");
+  // the rate charming_init read: asking the driver for it here took 1.3 ms,
+  // at times over 10
+  const int khz = charm_host::clock_khz();
   const double ms_per = khz > 0 ? 1.0 / khz : 0.0;
   double mx = 0, sum[6] = {0, 0, 0, 0, 0, 0};
   int busy = 0;
@@ -551,6 +556,7 @@ extern "C" int charming_jacobi2d_destroy(void* handle) {
   cudaFree(h->d_final);
   cudaFree(h->d_block_map);
   cudaFree(h->d_chare_of);
+  cudaFree(h->d_bc);
   cudaFree(h->d_sweep_ns);
   cudaFree(h->d_stage);
   cudaFree(h->d_pipe);

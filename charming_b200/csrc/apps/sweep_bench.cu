@@ -6,8 +6,8 @@
 // boundary and no halos move, so only the sweep is timed. For measuring and
 // profiling the sweep kernels; the results are not checked here (the chare
 // runs are, against the oracle).
-//   variant 0: multi-sweep pass, phase-split items (depth >= 2)
-//           1: multi-sweep pass, single-loop items (depth >= 2)
+//   variant 0: multi-sweep pass (depth >= 2)
+//           1: the same with the boundary tests in every step (depth >= 2)
 //           2: one sweep per pass, direct strip walker (depth 1)
 #include "suite.cuh"
 #include "jacobi_sweep.cuh"

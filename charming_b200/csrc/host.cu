@@ -30,6 +30,7 @@ struct HostRuntime {
   device_state ds{};
   std::vector<void*> dev_allocs;
   int* h_stop = nullptr;
+  unsigned long long* h_collect = nullptr;  // pinned: a run's status words, statistics and times
   int* d_stop = nullptr;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -134,6 +135,7 @@ void set_error_text(const std::string& s) { g_err = s; }
 bool initialised() { return g.inited; }
 cudaStream_t stream() { return g.stream; }
 const charming_info& info() { return g.inf; }
+int clock_khz() { return g.prop.clockRate; }
 int n_procs() { return g.world; }
 
 int ensure_init() {
@@ -200,19 +202,25 @@ int enqueue_status_latch(int* latch, cudaStream_t s) {
 }
 
 int collect_run(double kernel_ms) {
-  // the first error any of this launch's GPUs recorded
-  int ctrl_h[CTRL_WORDS];
+  // One synchronisation for everything a run left behind: status words of
+  // this launch's GPUs, statistics and times of its PEs, into pinned memory.
+  const int n_local = g.n_local;
+  const size_t ctrl_u64 = sizeof(int) * CTRL_WORDS / 8, n_ctrl = g.launch_ctrl.size();
+  unsigned long long *h_ctrl = g.h_collect, *st = h_ctrl + ctrl_u64 * n_ctrl, *tm = st + (size_t)n_local * N_STATS;
   cudaError_t e = cudaSuccess;
-  for (size_t d = 0; d < g.launch_ctrl.size(); d++) {
-    e = cudaMemcpy(ctrl_h, g.launch_ctrl[d], sizeof(ctrl_h), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(e, "read status");
+  for (size_t d = 0; d < n_ctrl && e == cudaSuccess; d++)
+    e = cudaMemcpyAsync(h_ctrl + ctrl_u64 * d, g.launch_ctrl[d], ctrl_u64 * 8, cudaMemcpyDeviceToHost, g.stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(st, g.ds.pe_stats, 8 * (size_t)n_local * N_STATS, cudaMemcpyDeviceToHost, g.stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(tm, g.ds.pe_times, 24 * (size_t)n_local, cudaMemcpyDeviceToHost, g.stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream);
+  if (e != cudaSuccess) return cuda_fail(e, "read status and statistics");
+  // the first error any of this launch's GPUs recorded
+  const int* ctrl_h = reinterpret_cast<const int*>(h_ctrl);
+  for (size_t d = 0; d < n_ctrl; d++) {
+    ctrl_h = reinterpret_cast<const int*>(h_ctrl + ctrl_u64 * d);
     if (ctrl_h[CTRL_STATUS] != 0) break;
   }
-  const int n_local = g.n_local;
-  std::vector<unsigned long long> st((size_t)n_local * N_STATS), tm((size_t)n_local * 3);
-  e = cudaMemcpy(st.data(), g.ds.pe_stats, st.size() * 8, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(tm.data(), g.ds.pe_times, tm.size() * 8, cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(e, "read stats");
   charming_stats s{};
   unsigned long long tmin = ~0ULL, tmax = 0, main_max = 0;
   for (int p = 0; p < n_local; p++) {
@@ -594,6 +602,9 @@ int charming_init_devices(const charming_config* cfg_in, const charming_devices*
                         "user heap blocks")))
       return rc;
   }
+  e = cudaHostAlloc(&g.h_collect, sizeof(int) * CTRL_WORDS * (size_t)launch_devs + 8ull * (N_STATS + 3) * n_local,
+                    cudaHostAllocDefault);
+  if (e != cudaSuccess) return cuda_fail(e, "run status buffer");
   e = cudaHostAlloc(&g.h_stop, 64, cudaHostAllocMapped);
   if (e != cudaSuccess) return cuda_fail(e, "host stop word");
   *g.h_stop = 0;
@@ -683,6 +694,8 @@ int charming_fini(void) {
   g.d_args_cap = 0;
   if (g.h_stop) cudaFreeHost(g.h_stop);
   g.h_stop = nullptr;
+  if (g.h_collect) cudaFreeHost(g.h_collect);
+  g.h_collect = nullptr;
   if (g.ev0) cudaEventDestroy(g.ev0);
   if (g.ev1) cudaEventDestroy(g.ev1);
   if (g.stream) cudaStreamDestroy(g.stream);

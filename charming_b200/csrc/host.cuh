@@ -18,6 +18,8 @@ bool initialised();
 
 cudaStream_t stream();
 const charming_info& info();
+// Nominal SM clock in kHz, read once by charming_init.
+int clock_khz();
 // Processes of the run (1 unless charming_init_devices was given world > 1).
 int n_procs();
 

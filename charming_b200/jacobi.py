@@ -124,7 +124,7 @@ class Jacobi2D:
         """One persistent launch that runs every problem to completion; returns
         its CUDA-event time in ms."""
         check(self.lib.charming_jacobi2d_run(self.h), "charming_jacobi2d_run")
-        return self.info()["last_run_ms"]
+        return self.rt.last_stats().kernel_ms
 
     def run_n(self, n_runs: int) -> float:
         """n_runs runs enqueued back to back and synchronised once (no host

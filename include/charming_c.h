@@ -340,7 +340,7 @@ int charming_sm_pingpong(int mode, int round_trips, double* oneway_ns, double* o
  * the chare sweep of examples/jacobi2d/jacobi2d.cu:327-334 as implemented
  * here): n_blocks (<= n_pes) PE-shaped thread blocks each run `passes`
  * passes of `depth` sweeps over their own w x h chare block. variant 0:
- * multi-sweep pass with phase-split items, 1: with single-loop items
+ * multi-sweep pass with no boundary tests in the steady steps, 1: with them in every step
  * (depth >= 2), 2: one
  * direct sweep per pass (depth 1). *ms receives the kernel time. */
 int charming_sweep_bench(int dtype, int w, int h, int depth, int passes, int n_blocks, int variant,
