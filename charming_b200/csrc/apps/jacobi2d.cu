@@ -2,11 +2,14 @@
 // (jacobi2d.cu:93-279) on this runtime, for many problems at once.
 //
 // Per chare and exchange ("pass"): receive one halo per neighbour, run the
-// pass's sweeps on the block (jacobi_sweep.cuh), then pack the new boundary
-// rows/columns straight into the neighbours' inbox rings (zero-copy
-// messages). Halos carry their pass number, which closes the reference's
-// ghost race (jacobi2d.cu:171-190 / :222): a halo of pass p lands in the
-// ghost zone of buffer p & 1. A pass is one sweep with ghost depth 1 (the
+// pass's sweeps on the block (jacobi_sweep.cuh), then write the new boundary
+// rows/columns straight into the neighbours' ghost zones and send each
+// neighbour a message that says so; thread 0 counts those messages by itself
+// (an inline entry method), the block runs when the last one is in. (With
+// refnum-tagged halos, corner messages or the bulk-copy sweep the values
+// travel inside the messages instead.) Halos carry their pass number, which
+// closes the reference's ghost race (jacobi2d.cu:171-190 / :222): a halo of
+// pass p lands in the ghost zone of buffer p & 1. A pass is one sweep with ghost depth 1 (the
 // reference's scheme) or up to `depth` sweeps with a ghost zone that deep,
 // corners included (temporal blocking: same arithmetic per point, fewer
 // exchanges and one read + one write of the block per pass).
@@ -30,7 +33,13 @@
 
 namespace {
 
-enum : int { EP_START = 0, EP_HALO = 1, EP_CONT = 2, EP_PARTIAL = 3, EP_DECISION = 4 };
+// NOTE, PARTIAL and DECISION are inline entry methods; PUMP is what the block
+// runs after one of them when its chare can go on, FRESH when the message is
+// the first of a request that the worker has not set up yet (serving).
+enum : int {
+  EP_START = 0, EP_HALO = 1, EP_CONT = 2, EP_NOTE = 3, EP_PARTIAL = 4, EP_DECISION = 5, EP_PUMP = 6,
+  EP_FRESH_NOTE = 7, EP_FRESH_PARTIAL = 8, EP_FRESH_DECISION = 9
+};
 enum : int { EP_POLL = 0 };  // server chare
 
 // g_app fields of this program.
@@ -300,8 +309,140 @@ struct halo_batch {
 };
 __shared__ halo_batch s_halos;
 
+// Halos go straight into the neighbours' ghost zones, with a note each. A
+// note's sender is at most one pass ahead of its receiver, so what it writes
+// (the ghost zone of buffer pass & 1) is neither read nor written by the pass
+// that the receiver may still be running.
+__device__ __forceinline__ bool puts_halos(const jac::chare_desc& d) {
+  return japp::halo_mode() == 0 && !japp::pipeline() && (d.depth == 1 || d.ext > 0);
+}
+
+// The puts of one batch, like halo_batch: rectangles of nr rows of nu units
+// (16-byte vectors, or single elements where a row of either side does not
+// start on a 16-byte boundary or is no whole number of vectors).
+struct put_batch {
+  int idx[4], pe[4], dirs[4];
+  size_t bytes[4];
+  const void* src[4];
+  void* dst[4];
+  int dst_pitch[4], nr[4], nu[4], unit[4];
+  int n;
+};
+__shared__ put_batch s_puts;
+
+// Rectangle k of the batch, by threads t of nt: the loads of four units are in
+// flight together; a thread's next unit is found by adding, not dividing.
+template <typename T, typename U>
+__device__ __forceinline__ void put_one(const put_batch& b, int k, int src_pitch, int t, int nt) {
+  constexpr int B = 4, W = sizeof(U) / sizeof(T);
+  const int nu = b.nu[k], total = b.nr[k] * nu, dst_pitch = b.dst_pitch[k];
+  const T* src = reinterpret_cast<const T*>(b.src[k]);
+  T* dst = reinterpret_cast<T*>(b.dst[k]);
+  int r = t / nu, x = t - r * nu;
+  const int dr = nt / nu, dx = nt - dr * nu;
+  for (int i = t; i < total; i += B * nt) {
+    U v[B];
+    int off[B];
+#pragma unroll
+    for (int q = 0; q < B; q++) {
+      if (i + q * nt < total) v[q] = *reinterpret_cast<const U*>(src + r * src_pitch + x * W);
+      off[q] = r * dst_pitch + x * W;
+      r += dr;
+      x += dx;
+      if (x >= nu) {
+        x -= nu;
+        r++;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < B; q++)
+      if (i + q * nt < total) *reinterpret_cast<U*>(dst + off[q]) = v[q];
+  }
+}
+
+// All rectangles of the batch, by threads t of nt: the warps are split among
+// them, so that their loads are in flight together. Out of line and lean:
+// every register that the callee keeps is saved by all threads (512 of them
+// with 80 registers each wait for 160 KB of local memory both ways).
 template <typename T>
-__device__ void send_halos(JBlock& c, const jac::chare_desc& d, int phase = 0) {
+__device__ __noinline__ void put_rects(int n, int src_pitch, int t, int nt) {
+  const put_batch& b = s_puts;
+  const int nw = nt >= 32 ? nt / 32 : 1, wi = nt >= 32 ? t / 32 : 0, groups = n < nw ? n : nw;
+  const int g = wi * groups / nw, w0 = (g * nw + groups - 1) / groups, w1 = ((g + 1) * nw + groups - 1) / groups;
+  const int tt = nt >= 32 ? t - 32 * w0 : t, tn = nt >= 32 ? 32 * (w1 - w0) : nt;
+  for (int k = g; k < n; k += groups) {
+    if (b.unit[k] > 1) put_one<T, typename jac::vec_of<T>::type>(b, k, src_pitch, tt, tn);
+    else put_one<T, T>(b, k, src_pitch, tt, tn);
+  }
+}
+
+// Writes the boundary regions of buf[cur] into the neighbours' ghost zones
+// (phase as in send_halos) and sends them their notes. The ring tickets are
+// taken by warp 0 while the other warps copy. All threads. On the headline
+// decomposition (2048 x 221 chares, 6 sweeps per pass) the halos of a pass
+// took about 105 us of 384 when they were packed into the ring, unpacked and
+// delivered to the block one by one, and take about 60 this way.
+template <typename T>
+__device__ void put_halos(JBlock& c, const jac::chare_desc& d, int phase) {
+  constexpr int V = jac::traits<T>::VEC;
+  const unsigned long long t0 = threadIdx.x == 0 ? pe_clock() : 0;
+  put_batch& b = s_puts;
+  if (threadIdx.x == 0) {
+    const jac::block_view<T> g = view<T>(d, c.cur);
+    int n = 0;
+    for (int dir = jac::TOP; dir <= jac::RIGHT; dir++) {
+      if (d.nbr[dir] < 0) continue;
+      if (phase == 1 && dir < jac::LEFT) continue;
+      if (phase == 2 && dir >= jac::LEFT) continue;
+      const jac::region e = jac::halo_edge(dir, d);
+      T* dst = reinterpret_cast<T*>(d.put[dir][c.pass & 1]);
+      const T* src = g.at(e.r0, e.c0);
+      const bool vec = e.nc % V == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
+      b.idx[n] = d.nbr[dir];
+      b.pe[n] = jproxy->loc_map[d.nbr[dir]];
+      b.dirs[n] = dir;
+      b.bytes[n] = sizeof(jac::halo_hdr);
+      b.src[n] = src;
+      b.dst[n] = dst;
+      b.dst_pitch[n] = d.put_pitch[dir];
+      b.unit[n] = vec ? V : 1;
+      b.nu[n] = e.nc / b.unit[n];
+      b.nr[n] = e.nr;
+      n++;
+    }
+    b.n = n;
+  }
+  __syncthreads();
+  const int n = b.n;
+  CHARM_PROF(if (threadIdx.x == 0) add_pe_cyc(5, pe_clock() - t0);)
+  const int w0 = blockDim.x >= 64 ? 32 : 0;  // warp 0 takes the tickets meanwhile
+  // A serving worker that has not seen its request yet fills its ghost zone
+  // when it does, with the same values as the first pass's halos: those are
+  // not put (they could be overwritten, or overwrite a later pass's).
+  if (n > 0 && (int)threadIdx.x >= w0 && !(japp::serving() && c.pass == 0))
+    put_rects<T>(n, d.pitch, (int)threadIdx.x - w0, (int)blockDim.x - w0);
+  charm::message* msg = charm::block_messages();
+  if (n > 0 && charm::alloc_user_msgs(msg, b.pe, b.bytes, n)) {
+    CHARM_PROF(if (threadIdx.x == 0) add_pe_cyc(3, pe_clock() - t0); const unsigned long long tp = pe_clock();)
+    for (int k = (int)threadIdx.x; k < n; k += (int)blockDim.x) {
+      jac::halo_hdr* hh = reinterpret_cast<jac::halo_hdr*>(msg[k].payload());
+      hh->dir = jac::opposite(b.dirs[k]);
+      hh->len = 0;
+      hh->pass = c.pass;
+      hh->gen = c.gen;
+    }
+    // publishes after a block barrier: the copies are done by then
+    jproxy->invoke_msgs(b.idx, EP_NOTE, msg, b.bytes, nullptr, n);
+    CHARM_PROF(if (threadIdx.x == 0) add_pe_cyc(4, pe_clock() - tp);)
+  }
+  if (threadIdx.x == 0) add_pe_cyc(1, pe_clock() - t0);
+}
+
+// Out of line, like the other paths that a chare with the default options
+// does not take (and the sweeps): inlined into the entry methods, their
+// registers were saved and restored by every thread on every delivery.
+template <typename T>
+__device__ __noinline__ void send_packed(JBlock& c, const jac::chare_desc& d, int phase) {
   const unsigned long long t0 = threadIdx.x == 0 ? pe_clock() : 0;
   halo_batch& b = s_halos;
   __syncthreads();  // every thread is done with the last batch's record
@@ -346,9 +487,15 @@ __device__ void send_halos(JBlock& c, const jac::chare_desc& d, int phase = 0) {
   if (threadIdx.x == 0) add_pe_cyc(1, pe_clock() - t0);
 }
 
+template <typename T>
+__device__ __forceinline__ void send_halos(JBlock& c, const jac::chare_desc& d, int phase) {
+  if (puts_halos(d)) put_halos<T>(c, d, phase);
+  else send_packed<T>(c, d, phase);
+}
+
 // Halo of pass hh->pass -> ghost zone of buf[pass & 1]. All threads.
 template <typename T>
-__device__ void unpack_halo(JBlock& c, const jac::chare_desc& d, const void* arg) {
+__device__ __noinline__ void unpack_halo(JBlock& c, const jac::chare_desc& d, const void* arg) {
   const jac::halo_hdr* hh = reinterpret_cast<const jac::halo_hdr*>(arg);
   T* vals = const_cast<T*>(reinterpret_cast<const T*>(reinterpret_cast<const char*>(arg) + sizeof(jac::halo_hdr)));
   jac::region gr = jac::halo_ghost(hh->dir, d);
@@ -421,9 +568,14 @@ __device__ void finish(JBlock& c, const jac::chare_desc& d) {
 // nothing of a completed request is in flight), without them a start that
 // went down the tree after its chare had finished can.
 template <typename T>
-__device__ int ensure_gen(JBlock& c, unsigned gen) {
+__device__ __noinline__ int set_up_gen(JBlock& c, unsigned gen);
+template <typename T>
+__device__ __forceinline__ int ensure_gen(JBlock& c, unsigned gen) {
+  return japp::serving() ? set_up_gen<T>(c, gen) : 1;
+}
+template <typename T>
+__device__ __noinline__ int set_up_gen(JBlock& c, unsigned gen) {
   using namespace charm::rt;
-  if (!japp::serving()) return 1;
   __shared__ int s_new;
   if (threadIdx.x == 0) s_new = gen > c.gen ? 1 : gen == c.gen ? 0 : -1;
   __syncthreads();
@@ -528,20 +680,40 @@ __device__ void em_poll(JServer& s, void* arg) {
   sproxy->invoke(0, EP_POLL);
 }
 
-__device__ void em_start(JBlock& c, void* arg) {
-  if (japp::dtype() == CHARMING_F32) em_start_t<float>(c, arg); else em_start_t<double>(c, arg);
+// Entry methods per grid type (the run registers those of its own: a test of
+// the type inside them would keep both types' registers alive).
+template <typename T>
+__device__ void em_start(JBlock& c, void* arg) { em_start_t<T>(c, arg); }
+template <typename T>
+__device__ void em_halo(JBlock& c, void* arg) { em_halo_t<T>(c, arg); }
+template <typename T>
+__device__ void em_cont(JBlock& c, void* arg) { em_cont_t<T>(c); }
+template <typename T>
+__device__ void em_pump(JBlock& c, void* arg) { pump<T>(c, c.desc); }
+// The first message of a request that this worker has not set up yet: set it
+// up, then take the message as the inline entry method would have.
+template <typename T, int In(JBlock&, void*)>
+__device__ void em_fresh(JBlock& c, void* arg) {
+  if (!ensure_gen<T>(c, msg_gen<In>(arg))) return;
+  __shared__ int s_next;
+  if (threadIdx.x == 0) s_next = In(c, arg);
+  __syncthreads();
+  const int next = s_next;
+  __syncthreads();
+  if (next == EP_PUMP) pump<T>(c, c.desc);
 }
-__device__ void em_halo(JBlock& c, void* arg) {
-  if (japp::dtype() == CHARMING_F32) em_halo_t<float>(c, arg); else em_halo_t<double>(c, arg);
-}
-__device__ void em_cont(JBlock& c, void* arg) {
-  if (japp::dtype() == CHARMING_F32) em_cont_t<float>(c); else em_cont_t<double>(c);
-}
-__device__ void em_partial(JBlock& c, void* arg) {
-  if (japp::dtype() == CHARMING_F32) em_partial_t<float>(c, arg); else em_partial_t<double>(c, arg);
-}
-__device__ void em_decision(JBlock& c, void* arg) {
-  if (japp::dtype() == CHARMING_F32) em_decision_t<float>(c, arg); else em_decision_t<double>(c, arg);
+template <typename T>
+__device__ void add_entry_methods() {  // in the order of EP_*
+  jproxy->add_entry_method<&em_start<T>>();
+  jproxy->add_entry_method<&em_halo<T>>();
+  jproxy->add_entry_method<&em_cont<T>>();
+  jproxy->add_inline_entry_method<&in_note>();
+  jproxy->add_inline_entry_method<&in_partial>();
+  jproxy->add_inline_entry_method<&in_decision>();
+  jproxy->add_entry_method<&em_pump<T>>();
+  jproxy->add_entry_method<&em_fresh<T, &in_note>>();
+  jproxy->add_entry_method<&em_fresh<T, &in_partial>>();
+  jproxy->add_entry_method<&em_fresh<T, &in_decision>>();
 }
 
 }  // namespace
@@ -550,11 +722,8 @@ __device__ void suite::jacobi2d_main(int pe) {
   if (threadIdx.x == 0) {
     for (int k = 0; k < 6; k++) s_pe_ns[k] = 0;
     jproxy = new charm::chare_proxy<JBlock>();
-    jproxy->add_entry_method<&em_start>();
-    jproxy->add_entry_method<&em_halo>();
-    jproxy->add_entry_method<&em_cont>();
-    jproxy->add_entry_method<&em_partial>();
-    jproxy->add_entry_method<&em_decision>();
+    if (japp::dtype() == CHARMING_F32) add_entry_methods<float>();
+    else add_entry_methods<double>();
     jproxy->create(japp::n_chares(), const_cast<int*>(japp::block_map()));
     if (!japp::serving()) {
       // each chare keeps its own descriptors (serving workers copy theirs

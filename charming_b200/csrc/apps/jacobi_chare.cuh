@@ -3,8 +3,9 @@
 //
 // State of a chare: `pass` exchanges done, `iter` sweeps done (buf[pass & 1]
 // holds u_iter), `sent` = last pass whose boundary was sent, got[p] = halos
-// received for the pass of parity p. A halo for pass k is unpacked into the
-// ghost zone of buf[k & 1] as soon as it arrives: pass k-1 reads only
+// received for the pass of parity p. A halo for pass k goes into the ghost
+// zone of buf[k & 1] as soon as it is there (its sender writes it, or it is
+// unpacked on arrival): pass k-1 reads only
 // buf[(k-1) & 1] and writes only the interior of buf[k & 1], and a neighbour
 // can be at most one pass ahead, so early halos need no stash (halo_mode 0).
 // halo_mode 1 tags halos with refnum = pass instead, which parks early ones
@@ -17,82 +18,56 @@
 // parked and may continue" to their caller instead of resuming it
 // themselves, so the call depth stays fixed whatever the message order.
 
-// All threads: record the decision of check m.check and pass it down the
-// tree. Returns 1 when the chare was parked on a decision (the caller then
-// runs pump()).
-template <typename T>
+// Thread 0: record the decision of check m.check and pass it down the tree.
+// Returns 1 when the chare was parked on a decision (the block then runs
+// pump()).
 __device__ int apply_decision(JBlock& c, const jac::chare_desc& d, const jac::decision_msg& m) {
-  __shared__ int s_resume;
-  if (threadIdx.x == 0) {
-    if (m.check > c.decided) c.decided = m.check;
-    if (m.stop && c.stop_check < 0) c.stop_check = m.check;
-    c.res0 = m.res0;
-    c.res_last = m.res;
-    c.checks = m.check + 1;
-    s_resume = c.waiting;
-    c.waiting = 0;
-  }
-  __syncthreads();
-  int resume = s_resume;
-  __syncthreads();
-  jac::decision_msg fwd = m;
+  if (m.check > c.decided) c.decided = m.check;
+  if (m.stop && c.stop_check < 0) c.stop_check = m.check;
+  c.res0 = m.res0;
+  c.res_last = m.res;
+  c.checks = m.check + 1;
+  const int resume = c.waiting;
+  c.waiting = 0;
   for (int k = 0; k < 2; k++) {
-    if (d.child[k] >= 0) jproxy->invoke(d.child[k], EP_DECISION, &fwd, sizeof(fwd));
+    if (d.child[k] >= 0) jproxy->invoke_single(d.child[k], EP_DECISION, &m, sizeof(m));
   }
   return resume;
 }
 
-// All threads: when this chare's partial and its children's are in, send
-// the sum up (fixed order: own, child 0, child 1) or decide at the root.
-// Thread 0 alone reads and writes the chare and builds the message; the
-// others only see it through shared memory. Returns apply_decision()'s
-// resume flag (0 when nothing was decided).
-template <typename T>
+// Thread 0: when this chare's partial and its children's are in, send the
+// sum up (fixed order: own, child 0, child 1) or decide at the root. Returns
+// apply_decision()'s resume flag (0 when nothing was decided). The tree's
+// messages are taken and sent by thread 0 alone: as block deliveries and
+// collective sends they were half of the time of small chares that check
+// their residual.
 __device__ int tree_try_forward(JBlock& c, const jac::chare_desc& d, int chk) {
-  __shared__ int s_act;
-  __shared__ jac::partial_msg s_pm;
-  __shared__ jac::decision_msg s_dm;
-  if (threadIdx.x == 0) {
-    s_act = 0;
-    bool complete = c.have_own && (d.child[0] < 0 || c.child_got[0]) &&
-                    (d.child[1] < 0 || c.child_got[1]);
-    if (complete) {
-      double t = c.own;
-      if (d.child[0] >= 0) t += c.child_val[0];
-      if (d.child[1] >= 0) t += c.child_val[1];
-      c.have_own = 0;
-      c.child_got[0] = c.child_got[1] = 0;
-      if (d.parent >= 0) {
-        s_pm.check = chk;
-        s_pm.slot = (d.rank - 1) % 2;
-        s_pm.gen = c.gen;
-        s_pm.pad = 0;
-        s_pm.value = t;
-        s_act = 1;
-      } else {
-        const jac::prob_desc& p = c.prob;
-        double nrm = sqrt(t);
-        s_dm.check = chk;
-        s_dm.gen = c.gen;
-        s_dm.pad = 0;
-        s_dm.res0 = (chk == 0) ? nrm : c.res0;
-        s_dm.res = nrm;
-        s_dm.stop = (p.tol > 0.0) && (s_dm.res0 == 0.0 || nrm <= p.tol * s_dm.res0) ? 1 : 0;
-        s_act = 2;
-      }
-    }
+  if (!(c.have_own && (d.child[0] < 0 || c.child_got[0]) && (d.child[1] < 0 || c.child_got[1]))) return 0;
+  double t = c.own;
+  if (d.child[0] >= 0) t += c.child_val[0];
+  if (d.child[1] >= 0) t += c.child_val[1];
+  c.have_own = 0;
+  c.child_got[0] = c.child_got[1] = 0;
+  if (d.parent >= 0) {
+    jac::partial_msg pm;
+    pm.check = chk;
+    pm.slot = (d.rank - 1) % 2;
+    pm.gen = c.gen;
+    pm.pad = 0;
+    pm.value = t;
+    jproxy->invoke_single(d.parent, EP_PARTIAL, &pm, sizeof(pm));
+    return 0;
   }
-  __syncthreads();
-  int act = s_act;
-  jac::partial_msg pm = s_pm;
-  jac::decision_msg dm = s_dm;
-  __syncthreads();
-  if (act == 1) {
-    jproxy->invoke(d.parent, EP_PARTIAL, &pm, sizeof(pm));
-  } else if (act == 2) {
-    return apply_decision<T>(c, d, dm);
-  }
-  return 0;
+  const jac::prob_desc& p = c.prob;
+  const double nrm = sqrt(t);
+  jac::decision_msg dm;
+  dm.check = chk;
+  dm.gen = c.gen;
+  dm.pad = 0;
+  dm.res0 = (chk == 0) ? nrm : c.res0;
+  dm.res = nrm;
+  dm.stop = (p.tol > 0.0) && (dm.res0 == 0.0 || nrm <= p.tol * dm.res0) ? 1 : 0;
+  return apply_decision(c, d, dm);
 }
 
 // All threads: one pass buf[pass&1] -> buf[(pass+1)&1], then the residual
@@ -115,12 +90,12 @@ __device__ void advance(JBlock& c, const jac::chare_desc& d) {
     if (resid) {
       c.own = part;
       c.have_own = 1;
+      // A decision taken here (at the tree root) cannot find this chare
+      // parked: it is sweeping. pump()'s loop re-examines the state anyway.
+      (void)tree_try_forward(c, d, chk);
     }
   }
   __syncthreads();
-  // A decision taken here (at the tree root) cannot find this chare parked:
-  // it is sweeping. pump()'s loop re-examines the state anyway.
-  if (resid) tree_try_forward<T>(c, d, chk);
 }
 
 // All threads: drive the chare as far as it can go without new messages:
@@ -260,39 +235,57 @@ __device__ void em_cont_t(JBlock& c) {
   pump<T>(c, d);
 }
 
-template <typename T>
-__device__ void em_partial_t(JBlock& c, void* arg) {
-  const jac::partial_msg* pm = reinterpret_cast<const jac::partial_msg*>(arg);
-  if (!ensure_gen<T>(c, pm->gen)) return;
-  if (c.done) return;
-  const jac::chare_desc& d = c.desc;
-  int chk = pm->check;
-  // Thread 0 checks and records the partial; the others learn the outcome
-  // after the barrier (reading child_got themselves would race with it).
-  __shared__ int s_ok;
-  if (threadIdx.x == 0) {
-    bool ok = CHARM_VERIFY(pm->slot == 0 || pm->slot == 1, CHARMING_ERR_APP, 5000 + pm->slot, c.i) &&
-              CHARM_VERIFY(d.child[pm->slot] >= 0 && !c.child_got[pm->slot], CHARMING_ERR_APP,
-                           6000 + pm->slot, c.i);
-    if (ok) {
-      c.child_val[pm->slot] = pm->value;
-      c.child_got[pm->slot] = 1;
-    }
-    s_ok = ok ? 1 : 0;
-  }
-  __syncthreads();
-  int ok = s_ok;
-  __syncthreads();
-  if (!ok) return;
-  if (tree_try_forward<T>(c, d, chk)) pump<T>(c, d);
+// ---- inline entry methods (thread 0) ----------------------------------------
+// A message of a newer request than the worker's (serving) goes to the block,
+// which sets the request up first; one of an older request is dropped.
+__device__ __forceinline__ int stale(const JBlock& c, unsigned gen, int fresh_ep) {
+  if (!japp::serving() || gen == c.gen) return 0;
+  return gen > c.gen ? fresh_ep : -1;
 }
 
-template <typename T>
-__device__ void em_decision_t(JBlock& c, void* arg) {
-  jac::decision_msg m = *reinterpret_cast<const jac::decision_msg*>(arg);
-  if (!ensure_gen<T>(c, m.gen)) return;
-  if (c.done) return;
-  const jac::chare_desc& d = c.desc;
-  __syncthreads();
-  if (apply_decision<T>(c, d, m)) pump<T>(c, d);
+// A neighbour's halo of hh->pass lies in the ghost zone: count it; the block
+// runs when the chare can go on (the conditions of pump()).
+__device__ int in_note(JBlock& c, void* arg) {
+  const jac::halo_hdr* hh = reinterpret_cast<const jac::halo_hdr*>(arg);
+  const int dir = hh->dir, pass = hh->pass;
+  if (const int s = stale(c, hh->gen, EP_FRESH_NOTE)) return s;
+  if (c.done) return -1;
+  if (!CHARM_VERIFY(dir >= 0 && dir < 4 && c.desc.nbr[dir] >= 0, CHARMING_ERR_APP, 1000 + dir, c.i) ||
+      !CHARM_VERIFY(pass == c.pass || pass == c.pass + 1, CHARMING_ERR_APP, 3000 + (pass - c.pass), c.i))
+    return -1;
+  c.got[pass & 1]++;
+  if (dir == jac::LEFT || dir == jac::RIGHT) c.gotx[pass & 1]++;
+  if (!c.started || c.waiting || c.sent < c.pass) return -1;  // (the start pumps; so does a decision)
+  if (c.desc.ext > 0 && c.sent_y < c.pass) return c.gotx[c.pass & 1] == c.nbx ? EP_PUMP : -1;
+  return c.got[c.pass & 1] == c.nbr_count ? EP_PUMP : -1;
 }
+
+__device__ int in_partial(JBlock& c, void* arg) {
+  const jac::partial_msg m = *reinterpret_cast<const jac::partial_msg*>(arg);
+  if (const int s = stale(c, m.gen, EP_FRESH_PARTIAL)) return s;
+  if (c.done) return -1;
+  const jac::chare_desc& d = c.desc;
+  if (!CHARM_VERIFY(m.slot == 0 || m.slot == 1, CHARMING_ERR_APP, 5000 + m.slot, c.i) ||
+      !CHARM_VERIFY(d.child[m.slot] >= 0 && !c.child_got[m.slot], CHARMING_ERR_APP, 6000 + m.slot, c.i))
+    return -1;
+  c.child_val[m.slot] = m.value;
+  c.child_got[m.slot] = 1;
+  return tree_try_forward(c, d, m.check) ? EP_PUMP : -1;
+}
+
+__device__ int in_decision(JBlock& c, void* arg) {
+  const jac::decision_msg m = *reinterpret_cast<const jac::decision_msg*>(arg);
+  if (const int s = stale(c, m.gen, EP_FRESH_DECISION)) return s;
+  if (c.done) return -1;
+  return apply_decision(c, c.desc, m) ? EP_PUMP : -1;
+}
+
+// The request generation a message of inline entry method In carries.
+template <int In(JBlock&, void*)>
+__device__ unsigned msg_gen(const void* arg);
+template <>
+__device__ unsigned msg_gen<in_note>(const void* arg) { return reinterpret_cast<const jac::halo_hdr*>(arg)->gen; }
+template <>
+__device__ unsigned msg_gen<in_partial>(const void* arg) { return reinterpret_cast<const jac::partial_msg*>(arg)->gen; }
+template <>
+__device__ unsigned msg_gen<in_decision>(const void* arg) { return reinterpret_cast<const jac::decision_msg*>(arg)->gen; }

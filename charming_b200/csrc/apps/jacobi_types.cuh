@@ -67,6 +67,10 @@ struct chare_desc {
   int pad_;
   void* buf[2];        // the two pitched grids, pointing at row 0 (ghost rows
                        // 1-D..0 lie before it)
+  // Sides TOP..RIGHT: the first ghost cell that a halo from this chare fills
+  // in its neighbour's grids, and the neighbour's pitch
+  void* put[4][2];
+  int put_pitch[4];
 };
 
 // The cells a halo from / to direction d covers, with the two-phase

@@ -661,6 +661,28 @@ __device__ void charm::send_reg_msg(int chare_id, int chare_idx, int ep_id, void
   if (threadIdx.x == 0) publish_msg(dst, t, m);
 }
 
+__device__ void charm::send_reg_msg_single(int chare_id, int chare_idx, int ep_id, const void* buf,
+    size_t payload_size, int dst_pe, int refnum) {
+  pe_state* ps = pes();
+  const unsigned long long bytes = envelope::alloc_size(msgtype::regular, payload_size);
+  unsigned long long t = 0;
+  unsigned char* m = reserve(dst_pe, bytes, &t);
+  if (m == nullptr) return;
+  envelope* env = reinterpret_cast<envelope*>(m);
+  env->type = msgtype::regular;
+  env->src_pe = charm::my_pe();
+  env->size = bytes;
+  regular_msg* rm = reinterpret_cast<regular_msg*>(m + sizeof(envelope));
+  rm->chare_id = chare_id;
+  rm->chare_idx = chare_idx;
+  rm->ep_id = ep_id;
+  rm->refnum = refnum;
+  if (buf && payload_size > 0) copy_cooperative(m + HDR, buf, payload_size, 0, 1);
+  ps->stats[ST_SENT]++;
+  ps->stats[ST_BYTES_SENT] += payload_size;
+  publish_msg(dst_pe, t, m);
+}
+
 __device__ bool charm::alloc_user_msg(message& msg, int dst_pe, size_t payload_size) {
   if (gpu_level()) return group_alloc_user_msgs(&msg, &dst_pe, &payload_size, 1);
   pe_state* ps = pes();
@@ -1307,6 +1329,22 @@ __device__ void stash_batch(chare_proxy_base* p, const stash_key* k, int ep, voi
   }
 }
 
+// Thread 0: runs entry method *ep of chare idx here if it is an inline one.
+// True when the delivery ended with it; else *ep is the entry method that the
+// block has to run.
+__device__ bool inline_done(pe_state* ps, chare_proxy_base* p, int idx, int* ep, void* arg) {
+  if (!p->inline_em(*ep)) return false;
+  const long long c0 = clock64();
+  const int next = p->run_inline(idx, *ep, arg);
+  ps->stats[ST_EM_CYC] += (unsigned long long)(clock64() - c0);
+  if (next < 0) {
+    if ((++ps->stats[ST_DELIVERED] & 15) == 0) stamp_progress(ps->my_pe);
+    return true;
+  }
+  *ep = next;
+  return false;
+}
+
 // Thread 0: decides what the block does next (pe_state d_* fields).
 __device__ void next_action() {
   pe_state* ps = pes();
@@ -1333,6 +1371,7 @@ __device__ void next_action() {
           ps->d_act = ACT_EXIT;
           return;
         }
+        if (inline_done(ps, p, idx, &ep, nullptr)) continue;
         ps->d_act = ACT_CALL_WAIT;
         ps->d_p = p;
         ps->d_idx = idx;
@@ -1375,16 +1414,25 @@ __device__ void next_action() {
       }
       const unsigned char* env = arena_of(slot) + (k->data_off % c_rt.stash_bytes);
       const regular_msg* rm = reinterpret_cast<const regular_msg*>(env + sizeof(envelope));
+      int ep = rm->ep_id;
+      if (inline_done(ps, p, k->chare_idx, &ep, const_cast<unsigned char*>(env) + HDR)) {
+        k->state = KEY_FREE;
+        ps->n_ready--;
+        stash_retire();
+        if (ps->revive_pending) break;  // it changed a refnum: look again first
+        continue;
+      }
       ps->d_act = ACT_CALL_STASH;
       ps->d_p = p;
       ps->d_idx = k->chare_idx;
-      ps->d_ep = rm->ep_id;
+      ps->d_ep = ep;
       ps->d_arg = const_cast<unsigned char*>(env) + HDR;
       ps->d_key = i;
       // (from the on-chip ready list; past RQ_MAX ready ones, one at a time)
       if (p->warp_em(rm->ep_id) && batching() && !ps->rq_over) stash_batch(p, k, rm->ep_id, ps->d_arg, i);
       return;
     }
+    if (ps->revive_pending) continue;
     // the inbox
     const int got = poll_inbox();
     if (got == 0) {
@@ -1396,6 +1444,12 @@ __device__ void next_action() {
     unsigned char* m = ring_cell(me, ps->head);
     const envelope* env = reinterpret_cast<const envelope*>(m);
     const regular_msg* rm = reinterpret_cast<const regular_msg*>(m + sizeof(envelope));
+#ifndef CHARMING_HOST_EMULATION
+    // the payload's first line comes with the header (an inline entry method
+    // reads it next); nothing waits for this load
+    unsigned int first;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(first) : "l"(m + HDR));
+#endif
     unsigned long long size = env->size;
     const int type = (int)env->type;
     ps->d_act = ACT_NONE;
@@ -1408,11 +1462,14 @@ __device__ void next_action() {
       if (p == nullptr || !p->valid_target(rm->chare_idx, rm->ep_id)) {
         set_error(CHARMING_ERR_BAD_TARGET, cid, rm->chare_idx);
       } else if (p->refnum_matches(rm->chare_idx, rm->refnum)) {
-        ps->d_act = ACT_CALL_RING;
-        ps->d_p = p;
-        ps->d_idx = rm->chare_idx;
-        ps->d_ep = rm->ep_id;
-        ps->d_arg = m + HDR;
+        int ep = rm->ep_id;
+        if (!inline_done(ps, p, rm->chare_idx, &ep, m + HDR)) {
+          ps->d_act = ACT_CALL_RING;
+          ps->d_p = p;
+          ps->d_idx = rm->chare_idx;
+          ps->d_ep = ep;
+          ps->d_arg = m + HDR;
+        }
         if (p->warp_em(rm->ep_id) && batching()) {
           // the first of a batch; warp 0 looks for more behind it
           ps->d_act = ACT_CALL_BATCH;

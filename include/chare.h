@@ -77,6 +77,8 @@ typedef bool (*proxy_call_fn)(chare_proxy_base* proxy, int idx, int ep, void* ar
 // One registered entry method with the lookup of its chare object: the
 // scheduler reaches an entry method with this one indirect call.
 typedef void (*em_entry_fn)(chare_proxy_base* proxy, int idx, void* arg);
+// The same for an inline entry method (add_inline_entry_method).
+typedef int (*em_inline_fn)(chare_proxy_base* proxy, int idx, void* arg);
 
 struct chare_proxy_base {
   int id;        // Chare array ID (registration order on this PE)
@@ -101,12 +103,22 @@ struct chare_proxy_base {
   // Entry methods 0..63 registered with add_warp_entry_method (bit ep): one
   // warp runs each of their deliveries.
   unsigned long long warp_ems;
+  // ... and those registered with add_inline_entry_method: run by the
+  // scheduler's deciding thread (their em_tab entry is an em_inline_fn).
+  unsigned long long inline_ems;
 
   __device__ chare_proxy_base() : id(-1), n_local(0), n_total(0), start_idx(-1),
   end_idx(-1), loc_map(nullptr), em_count(0), async_waits(nullptr),
-  refnum(nullptr), mismatches(nullptr), call_fn(nullptr), em_tab(nullptr), warp_ems(0) {}
+  refnum(nullptr), mismatches(nullptr), call_fn(nullptr), em_tab(nullptr), warp_ems(0), inline_ems(0) {}
 
   __device__ bool warp_em(int ep) const { return ep >= 0 && ep < 64 && ((warp_ems >> ep) & 1ULL); }
+
+  __device__ bool inline_em(int ep) const { return ep >= 0 && ep < 64 && ((inline_ems >> ep) & 1ULL); }
+  // Thread 0: runs inline entry method ep; the entry method that the block
+  // runs next on the same chare and argument, or -1.
+  __device__ int run_inline(int idx, int ep, void* arg) {
+    return reinterpret_cast<em_inline_fn>(em_tab[ep])(this, idx, arg);
+  }
 
   // Proxies come from the PE arena (shared memory when there is room), so
   // the scheduler's per-message reads of them stay on chip.
@@ -244,6 +256,29 @@ struct chare_proxy : chare_proxy_base {
     if (em_count == ep + 1) warp_ems |= 1ULL << ep;
   }
 
+  // Registers an entry method that the scheduler's deciding thread runs by
+  // itself, without the block (an extension, for small bookkeeping
+  // deliveries: a block delivery costs its barriers and the register frames
+  // of every thread). It must not synchronise and sends with invoke_single
+  // only. It returns the number of a block entry method of the same chare
+  // array that the block is to run next on this chare with the same
+  // argument, or -1 when the delivery is done. Single-threaded, like
+  // add_entry_method.
+  template <int Func(C&, void*)>
+  __device__ static int em_inline_entry(chare_proxy_base* base, int idx, void* arg) {
+    chare_proxy<C>* self = static_cast<chare_proxy<C>*>(base);
+    return Func(*(self->objects[idx - self->start_idx]), arg);
+  }
+  template <int Func(C&, void*)>
+  __device__ void add_inline_entry_method() {
+    if (em_tab == nullptr || em_count >= 64) {
+      detail::report_error(detail::ERR_TOO_MANY_EMS, id, em_count);
+      return;
+    }
+    inline_ems |= 1ULL << em_count;
+    em_tab[em_count++] = reinterpret_cast<em_entry_fn>(&chare_proxy<C>::template em_inline_entry<Func>);
+  }
+
   __device__ static bool call_static(chare_proxy_base* base, int idx, int ep, void* arg) {
     chare_proxy<C>* self = static_cast<chare_proxy<C>*>(base);
     self->em_tab[ep](base, idx, arg);
@@ -340,6 +375,16 @@ struct chare_proxy : chare_proxy_base {
       return;
     }
     send_reg_msg(id, idx, ep, buf, size, loc_map[idx], ref);
+  }
+
+  // Single-threaded: from inline entry methods, or one thread (thread 0) of
+  // a block entry method.
+  inline __device__ void invoke_single(int idx, int ep, const void* buf, size_t size, int ref = -1) {
+    if (idx < 0 || idx >= n_total) {
+      detail::report_error(detail::ERR_BAD_TARGET, id, idx);
+      return;
+    }
+    send_reg_msg_single(id, idx, ep, buf, size, loc_map[idx], ref);
   }
 
   inline __device__ void invoke_all(int ep) { invoke_all(ep, nullptr, 0); }

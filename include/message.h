@@ -116,6 +116,11 @@ struct alignas(ALIGN_SIZE) message {
 __device__ void send_reg_msg(int chare_id, int chare_idx, int ep_id, void* buf,
     size_t payload_size, int dst_pe, int refnum);
 __device__ void send_begin_term_msg();
+// Single-threaded send for inline entry methods (an extension, see
+// chare_proxy<C>::add_inline_entry_method): the calling thread, thread 0 of
+// the PE block, reserves, fills and publishes the message alone.
+__device__ void send_reg_msg_single(int chare_id, int chare_idx, int ep_id, const void* buf,
+    size_t payload_size, int dst_pe, int refnum);
 __device__ bool alloc_user_msg(message& msg, int dst_pe, size_t payload_size);
 __device__ void send_user_msg(int chare_id, int chare_idx, int ep_id,
     message& msg, size_t payload_size, int refnum);

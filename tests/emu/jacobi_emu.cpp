@@ -393,6 +393,10 @@ void send_reg_msg(int chare_id, int chare_idx, int ep, void* buf, size_t size, i
   if (threadIdx.x == 0) push(dst_pe, make_msg(msgtype::regular, chare_id, chare_idx, ep, refnum, buf, size));
   emu_sync(__FILE__, __LINE__);
 }
+void send_reg_msg_single(int chare_id, int chare_idx, int ep, const void* buf, size_t size, int dst_pe,
+    int refnum) {
+  push(dst_pe, make_msg(msgtype::regular, chare_id, chare_idx, ep, refnum, buf, size));
+}
 message* block_messages() { return me_pe().bmsgs; }
 // whether msg is in the block's shared array (filled by thread 0 alone)
 static bool block_shared(const message& msg) {
@@ -487,6 +491,12 @@ int classify(PE& pe) {
   if (!p->refnum_matches(rm->chare_idx, rm->refnum)) {
     pe.stash.push_back(Stashed{std::move(m), false});
     return ACT_IDLE;
+  }
+  if (p->inline_em(rm->ep_id)) {  // thread 0 alone; the block only if it says so
+    const int next = p->run_inline(rm->chare_idx, rm->ep_id, m.data() + 32);
+    g_progress++;
+    if (next < 0) return ACT_IDLE;
+    rm->ep_id = next;
   }
   return ACT_DELIVER;
 }

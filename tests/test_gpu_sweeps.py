@@ -46,3 +46,31 @@ def test_multi_sweep_pass_tile_edges(rt, dtype, depth):
         j.run()
         for p, g in enumerate(grids):
             assert same_bits(j.store(p), oracle(g, probs[p].max_sweeps)), sizes[p]
+
+
+# Halos written into the neighbours' ghost zones: side halos of whole vectors
+# on both sides, of odd columns or at odd offsets (element copies), one to four
+# neighbours, chares no deeper than the halo
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("depth", [1, 2, 3, 4, 7, 8])
+def test_put_halos_units(rt, dtype, depth):
+    rng = np.random.default_rng(100 + depth)
+    npdt = np.float64 if dtype == "f64" else np.float32
+    shapes = [(24, 24, 3, 3), (64, 48, 4, 2), (65, 47, 4, 2), (67, 50, 3, 3), (200, 9, 5, 1), (11, 160, 1, 7),
+              (301, 77, 2, 2), (512, 96, 1, 3)]
+    probs, grids = [], []
+    for nx, ny, px, py in shapes:
+        probs.append(Problem(nx, ny, 3 * depth + 2, px=px, py=py))
+        grids.append(rng.random((ny + 2, nx + 2)).astype(npdt))
+    with Jacobi2D(probs, dtype=dtype, depth=depth) as j:
+        for p, g in enumerate(grids):
+            j.load(p, g)
+        j.run()
+        for p, g in enumerate(grids):
+            assert same_bits(j.store(p), oracle(g, probs[p].max_sweeps)), shapes[p]
+        # the same again: nothing of the first run is left in the ghost zones
+        j.load(0, grids[0] * 0.5)
+        for p in range(1, len(grids)):
+            j.load(p, grids[p])
+        j.run()
+        assert same_bits(j.store(0), oracle((grids[0] * npdt(0.5)).astype(npdt), probs[0].max_sweeps))
