@@ -684,7 +684,7 @@ __device__ __forceinline__ double deep_item(const block_view<T>& in, const block
 // The same pass, computed by thread 0 alone for blocks under one warp, with
 // levels 1..L-1 kept as three-row rings in the block's scratch.
 template <typename T, bool RESID>
-__device__ double sweep_deep_simple(block_view<T> in, block_view<T> out, int w, int h, int L,
+__device__ __noinline__ double sweep_deep_simple(block_view<T> in, block_view<T> out, int w, int h, int L,
     int fixed) {
   if (threadIdx.x != 0) return 0.0;
   size_t cap = 0;
@@ -732,17 +732,29 @@ __device__ __noinline__ double sweep_deep_items(block_view<T> in, block_view<T> 
   constexpr int SS = 32 - 2 * E;        // vectors a strip owns
   const int nv = (w + V - 1) / V;
   const int n_strips = (nv + SS - 1) / SS;
-  // row runs: balance items over warps; each run at least 4L rows
-  int segs = 1, best = 0x7fffffff;
-  for (int sg = 1; sg <= 8; sg++) {
-    if (sg > 1 && h / sg < 4 * L) break;
-    int rounds = (n_strips * sg + nw - 1) / nw;
-    int cost = rounds * ((h + sg - 1) / sg + 2 * L);
-    if (cost < best) {
-      best = cost;
-      segs = sg;
+  // Row runs. More runs fill the warps but each streams 2L rows more than it
+  // stores. Cost of a split: its rows times the items that share an SM
+  // sub-partition's pipes (warps go to the four in turn) plus the items in
+  // sequence on the busiest warp (a step's latency is about one more item's
+  // worth of issue). Over the splits measured for 64^2 to 2048 x 221 blocks
+  // in both types (1 to 12 runs, 16 warps) its choice is within 1 % of the
+  // best one on average and 5 % at most; counting rounds of busy warps alone
+  // lost 5 % and up to 31 %. One lane per split: a loop over them in every
+  // thread took 2 us of a 256^2 block's 58.
+  unsigned long long key = ~0ULL;
+  {
+    const int sg = lane + 1;
+    if (sg <= 16 && (sg == 1 || h / sg >= 2 * L)) {
+      const int n = n_strips * sg, full = n / nw, rem = n - full * nw;
+      const int shared = full * ((nw + 3) / 4) + (rem + 3) / 4, chain = full + (rem > 0 ? 1 : 0);
+      key = ((unsigned long long)(unsigned)(shared + chain) * (unsigned)((h + sg - 1) / sg + 2 * L)) << 8 | (unsigned)sg;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long k = __shfl_xor_sync(0xffffffffu, key, o);
+      key = k < key ? k : key;
     }
   }
+  const int segs = (int)(key & 255);
   const int items = n_strips * segs;
   double acc = 0.0;
   for (int it = warp; it < items; it += nw) {
@@ -759,7 +771,7 @@ __device__ __noinline__ double sweep_deep_items(block_view<T> in, block_view<T> 
 // lean: steps that need no boundary or fill tests leave them out (false:
 // every step tests); same results bit for bit.
 template <typename T, bool RESID>
-__device__ __noinline__ double sweep_deep(block_view<T> in, block_view<T> out, int w, int h, int L,
+__device__ __forceinline__ double sweep_deep(block_view<T> in, block_view<T> out, int w, int h, int L,
     int fixed, bool lean = true) {
   if (blockDim.x < 32) return sweep_deep_simple<T, RESID>(in, out, w, h, L, fixed);
   using VT = typename vec_of<T>::type;
@@ -832,7 +844,7 @@ __device__ bool make_plan(int w, int nthreads, size_t smem_bytes, int tile_w_opt
 // waiting, so it never blocks the pipeline it feeds). Returns false (error
 // recorded) if a wait ran out.
 template <typename T, bool RESID>
-__device__ bool sweep_tma(block_view<T> in, block_view<T> out, int w, int h, void* smem,
+__device__ __noinline__ bool sweep_tma(block_view<T> in, block_view<T> out, int w, int h, void* smem,
     size_t smem_bytes, const tma_plan& P, double* acc_out) {
   constexpr int V = traits<T>::VEC;
   constexpr int H = V;  // halo elements each side of a slot row (16 bytes)
