@@ -25,6 +25,10 @@ struct JHandle {
   std::vector<int> chare_of;               // [prob offset + cy*px + cx] -> chare
   std::vector<size_t> chare_of_off;
   std::vector<int> px, py;
+  // all small device arrays lie in one allocation (d_small); results, done
+  // counter and phase timers side by side, zeroed together before a run
+  char* d_small = nullptr;
+  size_t zero_bytes = 0;
   jac::chare_desc* d_chares = nullptr;
   jac::prob_desc* d_probs = nullptr;
   jac::prob_result* d_results = nullptr;
@@ -59,65 +63,76 @@ __device__ __forceinline__ T* cell(const jac::chare_desc& d, int b, int r, int c
   return reinterpret_cast<T*>(d.buf[b]) + (size_t)r * d.pitch + jac::traits<T>::OFF - 1 + c;
 }
 
+// The three kernels below move whole grids between chare blocks and a
+// problem's global grid (or bc) and are bound by HBM: blocks of 64 x 4
+// threads, blockIdx.x the chare, its rows dealt over blockIdx.y and the 4
+// thread rows, no division per cell. With one block per chare (or a division
+// or four per cell) an 8192^2 load or store spent 0.9 and 0.3 ms in them.
+constexpr int GRID_TX = 64, GRID_TY = 4;
+
 // Initial state: boundary ring from bc (top/bottom rows include the corners),
 // interior 0; written to both buffers over the whole ghost zone wherever the
 // position lies on the global grid (ghost cells on the domain boundary must
-// hold boundary values for the multi-sweep pass). One block per chare.
+// hold boundary values for the multi-sweep pass).
 template <typename T>
-__global__ void init_kernel(const jac::chare_desc* ch, const jac::prob_desc* pr, const double* bc) {
-  const jac::chare_desc d = ch[blockIdx.x];
-  const jac::prob_desc p = pr[d.prob];
+__global__ void __launch_bounds__(GRID_TX * GRID_TY) init_kernel(const jac::chare_desc* ch, const jac::prob_desc* pr,
+    const double* bc) {
+  const jac::chare_desc& d = ch[blockIdx.x];
+  const jac::prob_desc& p = pr[d.prob];
   const double* b = bc + 4 * d.prob;
-  const int D = d.depth, W = d.w + 2 * D;
-  long long n = (long long)(d.h + 2 * D) * W;
-  for (long long x = threadIdx.x; x < n; x += blockDim.x) {
-    int r = (int)(x / W) + 1 - D, c = (int)(x % W) + 1 - D;
-    int gy = d.y0 + r, gx = d.x0 + c;
-    if (gy < 0 || gy > p.ny + 1 || gx < 0 || gx > p.nx + 1) continue;
-    double v = 0.0;
-    if (gy == 0) v = b[0];
-    else if (gy == p.ny + 1) v = b[1];
-    else if (gx == 0) v = b[2];
-    else if (gx == p.nx + 1) v = b[3];
-    *cell<T>(d, 0, r, c) = (T)v;
-    *cell<T>(d, 1, r, c) = (T)v;
+  const int D = d.depth, nx = p.nx, ny = p.ny;
+  for (int r = 1 - D + (int)(blockIdx.y * GRID_TY + threadIdx.y); r <= d.h + D; r += (int)(gridDim.y * GRID_TY)) {
+    const int gy = d.y0 + r;
+    if (gy < 0 || gy > ny + 1) continue;
+    T *a0 = cell<T>(d, 0, r, 0), *a1 = cell<T>(d, 1, r, 0);
+    for (int c = 1 - D + (int)threadIdx.x; c <= d.w + D; c += GRID_TX) {
+      const int gx = d.x0 + c;
+      if (gx < 0 || gx > nx + 1) continue;
+      const double v = gy == 0 ? b[0] : gy == ny + 1 ? b[1] : gx == 0 ? b[2] : gx == nx + 1 ? b[3] : 0.0;
+      a0[c] = a1[c] = (T)v;
+    }
   }
 }
 
 // Global grid (ny+2) x (nx+2) in `stage` -> blocks of one problem (whole
 // ghost zone, as init_kernel).
 template <typename T>
-__global__ void scatter_kernel(const jac::chare_desc* ch, const int* chare_of, int nx, int ny,
-    const T* stage) {
-  const jac::chare_desc d = ch[chare_of[blockIdx.x]];
-  const int D = d.depth, W = d.w + 2 * D;
-  long long n = (long long)(d.h + 2 * D) * W;
-  for (long long x = threadIdx.x; x < n; x += blockDim.x) {
-    int r = (int)(x / W) + 1 - D, c = (int)(x % W) + 1 - D;
-    int gy = d.y0 + r, gx = d.x0 + c;
-    if (gy < 0 || gy > ny + 1 || gx < 0 || gx > nx + 1) continue;
-    T v = stage[(size_t)gy * (nx + 2) + gx];
-    *cell<T>(d, 0, r, c) = v;
-    *cell<T>(d, 1, r, c) = v;
+__global__ void __launch_bounds__(GRID_TX * GRID_TY) scatter_kernel(const jac::chare_desc* ch, const int* chare_of,
+    int nx, int ny, const T* stage) {
+  const jac::chare_desc& d = ch[chare_of[blockIdx.x]];
+  const int D = d.depth;
+  for (int r = 1 - D + (int)(blockIdx.y * GRID_TY + threadIdx.y); r <= d.h + D; r += (int)(gridDim.y * GRID_TY)) {
+    const int gy = d.y0 + r;
+    if (gy < 0 || gy > ny + 1) continue;
+    T *__restrict__ a0 = cell<T>(d, 0, r, 0), *__restrict__ a1 = cell<T>(d, 1, r, 0);
+    const T* __restrict__ src = stage + (size_t)gy * (nx + 2) + d.x0;
+    const int c0 = max(1 - D, -d.x0), c1 = min(d.w + D, nx + 1 - d.x0);
+#pragma unroll 4
+    for (int c = c0 + (int)threadIdx.x; c <= c1; c += GRID_TX) a0[c] = a1[c] = src[c];
   }
 }
 
 // Blocks of one problem -> global grid: interior cells from their owner,
 // ring cells from the ghost ring of the edge chare next to them.
 template <typename T>
-__global__ void gather_kernel(const jac::chare_desc* ch, const int* chare_of, const int* final_buf,
-    int nx, int ny, int px, int py, T* stage) {
-  long long n = (long long)(nx + 2) * (ny + 2);
-  for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < n;
-       x += (long long)gridDim.x * blockDim.x) {
-    int gy = (int)(x / (nx + 2)), gx = (int)(x % (nx + 2));
-    int iy = min(max(gy - 1, 0), ny - 1), ix = min(max(gx - 1, 0), nx - 1);
-    int cy = jac::split_owner(ny, py, iy), cx = jac::split_owner(nx, px, ix);
-    int k = chare_of[cy * px + cx];
-    const jac::chare_desc& d = ch[k];
-    stage[x] = *cell<T>(d, final_buf[k], gy - d.y0, gx - d.x0);
+__global__ void __launch_bounds__(GRID_TX * GRID_TY) gather_kernel(const jac::chare_desc* ch, const int* chare_of,
+    const int* final_buf, int nx, int ny, int px, int py, T* stage) {
+  const int k = chare_of[blockIdx.x];
+  const jac::chare_desc& d = ch[k];
+  const int fb = final_buf[k];
+  const int r0 = d.cy == 0 ? 0 : 1, r1 = d.cy == py - 1 ? d.h + 1 : d.h;
+  const int c0 = d.cx == 0 ? 0 : 1, c1 = d.cx == px - 1 ? d.w + 1 : d.w;
+  for (int r = r0 + (int)(blockIdx.y * GRID_TY + threadIdx.y); r <= r1; r += (int)(gridDim.y * GRID_TY)) {
+    const T* __restrict__ src = cell<T>(d, fb, r, 0);
+    T* __restrict__ dst = stage + (size_t)(d.y0 + r) * (nx + 2) + d.x0;
+#pragma unroll 4
+    for (int c = c0 + (int)threadIdx.x; c <= c1; c += GRID_TX) dst[c] = src[c];
   }
 }
+
+// Enough blocks for a few waves whatever the number of chares.
+dim3 grid_blocks(int chares) { return dim3((unsigned)chares, (unsigned)std::min(64, std::max(1, 4096 / chares))); }
+constexpr dim3 grid_threads() { return dim3(GRID_TX, GRID_TY); }
 
 int fail(int code, const char* msg) {
   charm_host::set_error_text(msg);
@@ -178,25 +193,38 @@ extern "C" int charming_jacobi2d_create(const charming_jacobi_problem* probs, in
   }
   jac::place_buffers(&L, h->d_grid, (int)h->esz);
   h->chares = L.chares;
-  e = cudaMalloc(&h->d_chares, sizeof(jac::chare_desc) * nch);
-  if (e == cudaSuccess) e = cudaMalloc(&h->d_probs, sizeof(jac::prob_desc) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&h->d_results, sizeof(jac::prob_result) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&h->d_done, 64);
-  if (e == cudaSuccess) e = cudaMalloc(&h->d_final, sizeof(int) * nch);
-  if (e == cudaSuccess) e = cudaMalloc(&h->d_block_map, sizeof(int) * n_pes);
-  if (e == cudaSuccess) e = cudaMalloc(&h->d_chare_of, sizeof(int) * h->chare_of.size());
-  if (e == cudaSuccess) e = cudaMalloc(&h->d_sweep_ns, 64 * (size_t)n_pes);
-  std::vector<double> bc(4 * (size_t)n);
-  for (int p = 0; p < n; p++)
-    for (int k = 0; k < 4; k++) bc[4 * (size_t)p + k] = probs[p].bc[k];
-  if (e == cudaSuccess) e = cudaMalloc(&h->d_bc, sizeof(double) * bc.size());
-  if (e == cudaSuccess) e = cudaMemcpy(h->d_bc, bc.data(), sizeof(double) * bc.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(h->d_chares, h->chares.data(), sizeof(jac::chare_desc) * nch, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(h->d_probs, pd.data(), sizeof(jac::prob_desc) * n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(h->d_results, 0, sizeof(jac::prob_result) * n);
-  if (e == cudaSuccess) e = cudaMemset(h->d_final, 0, sizeof(int) * nch);
-  if (e == cudaSuccess) e = cudaMemcpy(h->d_block_map, h->block_map.data(), sizeof(int) * n_pes, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(h->d_chare_of, h->chare_of.data(), sizeof(int) * h->chare_of.size(), cudaMemcpyHostToDevice);
+  {
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+      const size_t o = at;
+      at += (bytes + 255) / 256 * 256;
+      return o;
+    };
+    const size_t o_res = take(sizeof(jac::prob_result) * (size_t)n), o_done = take(64),
+                 o_ns = take(64 * (size_t)n_pes);
+    h->zero_bytes = at;
+    const size_t o_final = take(sizeof(int) * (size_t)nch), o_ch = take(sizeof(jac::chare_desc) * (size_t)nch),
+                 o_pr = take(sizeof(jac::prob_desc) * (size_t)n), o_map = take(sizeof(int) * (size_t)n_pes),
+                 o_of = take(sizeof(int) * h->chare_of.size()), o_bc = take(4 * sizeof(double) * (size_t)n);
+    std::vector<char> img(at, 0);
+    memcpy(&img[o_ch], h->chares.data(), sizeof(jac::chare_desc) * (size_t)nch);
+    memcpy(&img[o_pr], pd.data(), sizeof(jac::prob_desc) * (size_t)n);
+    memcpy(&img[o_map], h->block_map.data(), sizeof(int) * (size_t)n_pes);
+    memcpy(&img[o_of], h->chare_of.data(), sizeof(int) * h->chare_of.size());
+    for (int p = 0; p < n; p++) memcpy(&img[o_bc + 32 * (size_t)p], probs[p].bc, 32);
+    e = cudaMalloc(&h->d_small, at);
+    if (e == cudaSuccess) e = cudaMemcpy(h->d_small, img.data(), at, cudaMemcpyHostToDevice);
+    char* d = h->d_small;
+    h->d_results = reinterpret_cast<jac::prob_result*>(d + o_res);
+    h->d_done = reinterpret_cast<unsigned long long*>(d + o_done);
+    h->d_sweep_ns = reinterpret_cast<unsigned long long*>(d + o_ns);
+    h->d_final = reinterpret_cast<int*>(d + o_final);
+    h->d_chares = reinterpret_cast<jac::chare_desc*>(d + o_ch);
+    h->d_probs = reinterpret_cast<jac::prob_desc*>(d + o_pr);
+    h->d_block_map = reinterpret_cast<int*>(d + o_map);
+    h->d_chare_of = reinterpret_cast<int*>(d + o_of);
+    h->d_bc = reinterpret_cast<double*>(d + o_bc);
+  }
   if (e == cudaSuccess) e = cudaHostAlloc(&h->h_params, sizeof(suite::app_params), cudaHostAllocDefault);
   if (e == cudaSuccess) e = cudaEventCreate(&h->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&h->ev1);
@@ -240,12 +268,33 @@ extern "C" int charming_jacobi2d_init(void* handle) {
   JHandle* h = reinterpret_cast<JHandle*>(handle);
   if (!h) return CHARMING_ERR_CONFIG;
   cudaStream_t s = charm_host::stream();
-  if (h->esz == 8) init_kernel<double><<<h->n_chares, 256, 0, s>>>(h->d_chares, h->d_probs, h->d_bc);
-  else init_kernel<float><<<h->n_chares, 256, 0, s>>>(h->d_chares, h->d_probs, h->d_bc);
+  if (h->esz == 8) init_kernel<double><<<grid_blocks(h->n_chares), grid_threads(), 0, s>>>(h->d_chares, h->d_probs, h->d_bc);
+  else init_kernel<float><<<grid_blocks(h->n_chares), grid_threads(), 0, s>>>(h->d_chares, h->d_probs, h->d_bc);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemsetAsync(h->d_final, 0, sizeof(int) * h->n_chares, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   return check_cuda(e, "jacobi2d init");
+}
+
+// Device-side work of load (staged grid -> chare blocks) and store (chare
+// blocks -> staged grid) on stream s, without the host copies.
+static void enqueue_scatter(JHandle* h, int prob, const void* stage, cudaStream_t s) {
+  const charming_jacobi_problem& q = h->probs[prob];
+  const dim3 g = grid_blocks(h->px[prob] * h->py[prob]), t = grid_threads();
+  const int* co = h->d_chare_of + h->chare_of_off[prob];
+  if (h->esz == 8) scatter_kernel<double><<<g, t, 0, s>>>(h->d_chares, co, q.nx, q.ny, (const double*)stage);
+  else scatter_kernel<float><<<g, t, 0, s>>>(h->d_chares, co, q.nx, q.ny, (const float*)stage);
+}
+static void enqueue_gather(JHandle* h, int prob, void* stage, cudaStream_t s) {
+  const charming_jacobi_problem& q = h->probs[prob];
+  const dim3 g = grid_blocks(h->px[prob] * h->py[prob]), t = grid_threads();
+  const int* co = h->d_chare_of + h->chare_of_off[prob];
+  if (h->esz == 8)
+    gather_kernel<double><<<g, t, 0, s>>>(h->d_chares, co, h->d_final, q.nx, q.ny, h->px[prob], h->py[prob],
+                                          (double*)stage);
+  else
+    gather_kernel<float><<<g, t, 0, s>>>(h->d_chares, co, h->d_final, q.nx, q.ny, h->px[prob], h->py[prob],
+                                         (float*)stage);
 }
 
 static int ensure_stage(JHandle* h, size_t bytes) {
@@ -268,11 +317,8 @@ extern "C" int charming_jacobi2d_load(void* handle, int prob, const void* host_g
   if (rc) return rc;
   cudaStream_t s = charm_host::stream();
   cudaError_t e = cudaMemcpyAsync(h->d_stage, host_grid, bytes, cudaMemcpyHostToDevice, s);
-  int nc = h->px[prob] * h->py[prob];
-  const int* co = h->d_chare_of + h->chare_of_off[prob];
   if (e == cudaSuccess) {
-    if (h->esz == 8) scatter_kernel<double><<<nc, 256, 0, s>>>(h->d_chares, co, q.nx, q.ny, (const double*)h->d_stage);
-    else scatter_kernel<float><<<nc, 256, 0, s>>>(h->d_chares, co, q.nx, q.ny, (const float*)h->d_stage);
+    enqueue_scatter(h, prob, h->d_stage, s);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(h->d_final, 0, sizeof(int) * h->n_chares, s);
@@ -289,14 +335,7 @@ extern "C" int charming_jacobi2d_store(void* handle, int prob, void* host_grid) 
   int rc = ensure_stage(h, bytes);
   if (rc) return rc;
   cudaStream_t s = charm_host::stream();
-  const int* co = h->d_chare_of + h->chare_of_off[prob];
-  int blocks = (int)std::min<size_t>((cells + 255) / 256, 4096);
-  if (h->esz == 8)
-    gather_kernel<double><<<blocks, 256, 0, s>>>(h->d_chares, co, h->d_final, q.nx, q.ny,
-        h->px[prob], h->py[prob], (double*)h->d_stage);
-  else
-    gather_kernel<float><<<blocks, 256, 0, s>>>(h->d_chares, co, h->d_final, q.nx, q.ny,
-        h->px[prob], h->py[prob], (float*)h->d_stage);
+  enqueue_gather(h, prob, h->d_stage, s);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(host_grid, h->d_stage, bytes, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -305,9 +344,7 @@ extern "C" int charming_jacobi2d_store(void* handle, int prob, void* host_grid) 
 
 // Work of one run on stream s: counters, program parameters, scheduler.
 static int enqueue_run(JHandle* h, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(h->d_done, 0, 64, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(h->d_results, 0, sizeof(jac::prob_result) * h->probs.size(), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(h->d_sweep_ns, 0, 64 * h->block_map.size(), s);
+  cudaError_t e = cudaMemsetAsync(h->d_small, 0, h->zero_bytes, s);
   if (e == cudaSuccess)
     e = cudaMemcpyToSymbolAsync(g_app, h->h_params, sizeof(suite::app_params), 0,
                                 cudaMemcpyHostToDevice, s);
@@ -383,28 +420,6 @@ extern "C" int charming_jacobi2d_run_n(void* handle, int n_runs, double* total_m
   if (e != cudaSuccess) return check_cuda(e, "jacobi2d run status");
   rc = charm_host::collect_run(h->last_ms);
   return latch[0] ? latch[0] : rc;
-}
-
-// Device-side work of load (staged grid -> chare blocks) and store (chare
-// blocks -> staged grid) on stream s, without the host copies.
-static void enqueue_scatter(JHandle* h, int prob, const void* stage, cudaStream_t s) {
-  const charming_jacobi_problem& q = h->probs[prob];
-  const int nc = h->px[prob] * h->py[prob];
-  const int* co = h->d_chare_of + h->chare_of_off[prob];
-  if (h->esz == 8) scatter_kernel<double><<<nc, 256, 0, s>>>(h->d_chares, co, q.nx, q.ny, (const double*)stage);
-  else scatter_kernel<float><<<nc, 256, 0, s>>>(h->d_chares, co, q.nx, q.ny, (const float*)stage);
-}
-static void enqueue_gather(JHandle* h, int prob, void* stage, cudaStream_t s) {
-  const charming_jacobi_problem& q = h->probs[prob];
-  const size_t cells = (size_t)(q.nx + 2) * (q.ny + 2);
-  const int* co = h->d_chare_of + h->chare_of_off[prob];
-  const int blocks = (int)std::min<size_t>((cells + 255) / 256, 4096);
-  if (h->esz == 8)
-    gather_kernel<double><<<blocks, 256, 0, s>>>(h->d_chares, co, h->d_final, q.nx, q.ny, h->px[prob],
-                                                 h->py[prob], (double*)stage);
-  else
-    gather_kernel<float><<<blocks, 256, 0, s>>>(h->d_chares, co, h->d_final, q.nx, q.ny, h->px[prob],
-                                                h->py[prob], (float*)stage);
 }
 
 static int ensure_pipe(JHandle* h, size_t bytes) {
@@ -549,15 +564,7 @@ extern "C" int charming_jacobi2d_destroy(void* handle) {
   if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
   if (h->graph) cudaGraphDestroy(h->graph);
   cudaFree(h->d_grid);
-  cudaFree(h->d_chares);
-  cudaFree(h->d_probs);
-  cudaFree(h->d_results);
-  cudaFree(h->d_done);
-  cudaFree(h->d_final);
-  cudaFree(h->d_block_map);
-  cudaFree(h->d_chare_of);
-  cudaFree(h->d_bc);
-  cudaFree(h->d_sweep_ns);
+  cudaFree(h->d_small);
   cudaFree(h->d_stage);
   cudaFree(h->d_pipe);
   cudaFree(h->d_latch);
