@@ -22,6 +22,8 @@
 #include "jacobi_sweep.cuh"
 #include "../host.cuh"
 
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 namespace {
@@ -64,38 +66,197 @@ int scratch_on_current_device(void** out, int* sms) {
   return CHARMING_OK;
 }
 
-// One sweep src -> dst over the interior of a row-major (ny+2) x (nx+2)
-// grid; the boundary ring of dst is already in place.
+// L sweeps src -> dst in one pass over a row-major (ny+2) x (nx+2) grid, the
+// boundary ring included (it is copied), with the chares' wavefront
+// (jac::deep_step): a warp streams the rows of one item, a strip of 32
+// vectors times a run of rows, and keeps the levels between in registers.
+// Rows have any alignment here: ALIGNED (16-byte aligned grids whose rows are
+// whole vectors) loads and stores vectors, else element by element. The next
+// NA_U rows are in flight in registers. FIX: the item's levels can meet the
+// boundary ring. The grids stay in L2; small ones are bound by the launch and
+// the chain of a warp's rows, large ones by instruction issue. 254^2 FP64, 20
+// sweeps: 96 us with one launch per sweep (two copies, a 64-bit division per
+// point); 2046^2 FP32, 100 sweeps: 1870 us.
+constexpr int NA_U = 4;
+
+template <typename T, int L, bool ALIGNED, bool FIX>
+__device__ __forceinline__ void noalloc_item(const T* __restrict__ src, T* __restrict__ dst, int nx, int ny,
+    int own0, int nown, int r0, int r1) {
+  constexpr int V = jac::traits<T>::VEC, E = (L + V - 1) / V, LH = (L + 1) / 2, U = NA_U;
+  const int lane = (int)(threadIdx.x & 31), v = own0 - E + lane, col0 = v * V, W = nx + 2;
+  jac::deep_lane<T> ln;
+  ln.v = v;
+  ln.col0 = col0;
+  ln.own = lane >= E && lane < E + nown;
+  ln.anyfix = false;
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    ln.fixc[k] = col0 + k == 0 || col0 + k == nx + 1;
+    ln.inw[k] = false;
+  }
+  ln.fix_r0 = 0;
+  ln.fix_r1 = ny + 1;
+  const int qs = r0 - L, qe = r1 - 1 + L;
+  // columns and rows off the grid: its nearest ones, never used by a result
+  int off[V];
+#pragma unroll
+  for (int k = 0; k < V; k++) off[k] = min(max(col0 + k, 0), nx + 1);
+  const int voff = min(max(col0, 0), ALIGNED ? W - V : 0);
+  T buf[U][V], x[V];
+  int next = qs;
+  auto load = [&](int u) {
+    const T* row = src + (size_t)min(max(next, 0), ny + 1) * W;
+    next++;
+    if (ALIGNED) {
+      const typename jac::vec_of<T>::type t = *reinterpret_cast<const typename jac::vec_of<T>::type*>(row + voff);
+      jac::vec_to<T>(t, buf[u]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < V; k++) buf[u][k] = row[off[k]];
+    }
+  };
+#pragma unroll
+  for (int u = 0; u < U; u++) load(u);
+  jac::deep_state<T, L> S;
+#pragma unroll
+  for (int l = 0; l < L; l++)
+#pragma unroll
+    for (int k = 0; k < V; k++) S.P[l][k] = S.X[l][k] = (T)0;
+#pragma unroll
+  for (int k = 0; k < V; k++) S.D[k] = 0.0;
+  double acc = 0.0;
+  T* op = dst + (size_t)r0 * W + col0;
+  const int nput = ln.own ? W - col0 : 0;
+  int q = qs;
+  // the first steps of the fill work on the lower half of the levels only
+  constexpr int F = 2 * LH / U * U;
+#pragma unroll 1
+  for (; q < qs + F; q += U) {
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+#pragma unroll
+      for (int k = 0; k < V; k++) x[k] = buf[u][k];
+      load(u);
+      jac::deep_step<T, false, L, LH, FIX>(S, x, q + u, ln, r0, r1, acc);
+    }
+  }
+#pragma unroll 1
+  for (; q <= qe; q += U) {
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+#pragma unroll
+      for (int k = 0; k < V; k++) x[k] = buf[u][k];
+      load(u);
+      jac::deep_step<T, false, L, L, FIX>(S, x, q + u, ln, r0, r1, acc);
+      const bool full = q + u >= qs + 2 * L && q + u <= qe;  // a row r0 .. r1 - 1 is complete
+      const int n = full ? nput : 0;
+      if (ALIGNED) {
+        jac::put_vec(op, x, n);
+      } else {
+#pragma unroll
+        for (int k = 0; k < V; k++)
+          if (k < n) op[k] = x[k];
+      }
+      op += full ? W : 0;
+    }
+  }
+}
+
+template <typename T, int L, bool ALIGNED>
+__global__ void __launch_bounds__(128) noalloc_pass_kernel(const T* __restrict__ src, T* __restrict__ dst, int nx,
+    int ny, int strips, int run_rows, int items) {
+  constexpr int V = jac::traits<T>::VEC, E = (L + V - 1) / V, SS = 32 - 2 * E;
+  const int item = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (item >= items) return;
+  const int nv = (nx + 2 + V - 1) / V, own0 = item % strips * SS, nown = min(SS, nv - own0);
+  const int r0 = item / strips * run_rows, r1 = min(ny + 2, r0 + run_rows);
+  const bool edge = own0 - E <= 0 || (own0 + nown + E) * V > nx + 1 || r0 - L <= 0 || r1 - 1 + L >= ny + 1;
+  if (edge) noalloc_item<T, L, ALIGNED, true>(src, dst, nx, ny, own0, nown, r0, r1);
+  else noalloc_item<T, L, ALIGNED, false>(src, dst, nx, ny, own0, nown, r0, r1);
+}
+
+constexpr int NA_LMAX = 8;
+
+// One pass of L sweeps: how the rows are split, and its cost in SM cycles. A
+// pass costs its launch and first loads (5000), then its rows: a warp's step
+// through one level takes 55 cycles alone and 38 of its SM sub-partition's
+// when several warps share it. (Measured on a B200 to within a quarter; the
+// choice only needs their ratio.)
+struct pass_plan {
+  int run_rows, strips, items;
+  double cycles;
+};
 template <typename T>
-__global__ void __launch_bounds__(256) noalloc_sweep_kernel(const T* __restrict__ src,
-    T* __restrict__ dst, int nx, int ny) {
-  const long long W = nx + 2;
-  const long long n = (long long)nx * ny;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    long long r = i / nx + 1, c = i % nx + 1;
-    const T* m = src + r * W + c;
-    dst[r * W + c] = jac::stencil(m[0], m[-1], m[1], m[-W], m[W]);
+pass_plan plan_pass(int L, int nx, int ny, int sms) {
+  constexpr int V = jac::traits<T>::VEC;
+  const int E = (L + V - 1) / V, SS = 32 - 2 * E, rows = ny + 2;
+  const int strips = ((nx + 2 + V - 1) / V + SS - 1) / SS;
+  pass_plan best{0, strips, 0, 1e300};
+  for (int R = 4; R <= 128; R += R < 16 ? 2 : R < 64 ? 8 : 32) {
+    const long long items = (long long)strips * ((rows + R - 1) / R);
+    const double per_part = std::ceil((double)items / (4.0 * sms));
+    const double c = 5000.0 + (double)(std::min(R, rows) + 2 * L) * L * std::max(55.0, 38.0 * per_part);
+    if (c < best.cycles) best = pass_plan{R, strips, (int)items, c};
+    if (R >= rows) break;
+  }
+  return best;
+}
+
+template <typename T, int L>
+void launch_pass(const T* src, T* dst, int nx, int ny, const pass_plan& p, bool aligned, int sms) {
+  // few items: blocks of one warp, so that they spread over the SMs
+  const int threads = p.items <= 4 * sms ? 32 : p.items <= 8 * sms ? 64 : 128;
+  const int blocks = (int)(((long long)p.items * 32 + threads - 1) / threads);
+  if (aligned) noalloc_pass_kernel<T, L, true><<<blocks, threads, 0, 0>>>(src, dst, nx, ny, p.strips, p.run_rows, p.items);
+  else noalloc_pass_kernel<T, L, false><<<blocks, threads, 0, 0>>>(src, dst, nx, ny, p.strips, p.run_rows, p.items);
+}
+template <typename T>
+void launch_pass_of(int L, const T* src, T* dst, int nx, int ny, const pass_plan& p, bool aligned, int sms) {
+  switch (L) {
+    case 1: return launch_pass<T, 1>(src, dst, nx, ny, p, aligned, sms);
+    case 2: return launch_pass<T, 2>(src, dst, nx, ny, p, aligned, sms);
+    case 3: return launch_pass<T, 3>(src, dst, nx, ny, p, aligned, sms);
+    case 4: return launch_pass<T, 4>(src, dst, nx, ny, p, aligned, sms);
+    case 5: return launch_pass<T, 5>(src, dst, nx, ny, p, aligned, sms);
+    case 6: return launch_pass<T, 6>(src, dst, nx, ny, p, aligned, sms);
+    case 7: return launch_pass<T, 7>(src, dst, nx, ny, p, aligned, sms);
+    default: return launch_pass<T, 8>(src, dst, nx, ny, p, aligned, sms);
   }
 }
 
 template <typename T>
 int run_sweeps(int nx, int ny, int sweeps, const T* in, T* out, T* scratch, int sms) {
   const size_t bytes = ((size_t)nx + 2) * ((size_t)ny + 2) * sizeof(T);
-  // Both buffers start as the input (boundary ring included); the first
-  // source is picked so that the last sweep writes `out`.
-  cudaError_t e = cudaMemcpyAsync(out, in, bytes, cudaMemcpyDeviceToDevice, 0);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(scratch, in, bytes, cudaMemcpyDeviceToDevice, 0);
-  T* a = (sweeps % 2 == 0) ? out : scratch;
-  T* b = (a == out) ? scratch : out;
-  const long long pts = (long long)nx * ny;
-  const int blocks = (int)std::min<long long>((pts + 255) / 256, (long long)sms * 8);
-  for (int s = 0; s < sweeps && e == cudaSuccess; s++) {
-    noalloc_sweep_kernel<T><<<blocks, 256, 0, 0>>>(a, b, nx, ny);
-    e = cudaGetLastError();
-    T* t = a;
-    a = b;
-    b = t;
+  cudaError_t e = cudaSuccess;
+  if (sweeps == 0) {
+    e = cudaMemcpyAsync(out, in, bytes, cudaMemcpyDeviceToDevice, 0);
+  } else {
+    // passes of the length that costs least per sweep, as even as they go:
+    // the first `longer` of them are one sweep longer than the rest
+    int best = 1;
+    double cost = 1e300;
+    pass_plan plans[NA_LMAX + 1];
+    for (int L = 1; L <= NA_LMAX; L++) {
+      plans[L] = plan_pass<T>(L, nx, ny, sms);
+      const double c = plans[L].cycles * ((sweeps + L - 1) / L);
+      if (c < cost) {
+        cost = c;
+        best = L;
+      }
+    }
+    const int n = (sweeps + best - 1) / best, base = sweeps / n, longer = sweeps % n;
+    const bool aligned = ((size_t)nx + 2) * sizeof(T) % 16 == 0 &&
+                         ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+    // the last pass writes `out`; every pass writes its whole target, ring
+    // included
+    const T* src = in;
+    for (int k = 0; k < n && e == cudaSuccess; k++) {
+      T* dst = (n - 1 - k) % 2 == 0 ? out : scratch;
+      const int L = base + (k < longer ? 1 : 0);
+      launch_pass_of<T>(L, src, dst, nx, ny, plans[L], aligned, sms);
+      e = cudaGetLastError();
+      src = dst;
+    }
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(0);
   if (e != cudaSuccess) return charm_host::cuda_fail(e, "jacobi2d noalloc sweeps");

@@ -74,3 +74,30 @@ def test_put_halos_units(rt, dtype, depth):
             j.load(p, grids[p])
         j.run()
         assert same_bits(j.store(0), oracle((grids[0] * npdt(0.5)).astype(npdt), probs[0].max_sweeps))
+
+
+# charming_jacobi2d_sweeps_noalloc: pass lengths 1..8 and their splits, vector
+# rows and element rows (odd widths, grids one element off a 16-byte
+# boundary), strip and row-run remainders, the smallest and largest grids
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("nx,ny,sweeps,shift", [
+    (1, 1, 3, 0), (2, 5, 1, 0), (3, 2, 9, 1), (6, 300, 7, 0), (301, 4, 8, 0), (46, 33, 2, 1), (54, 61, 13, 0),
+    (110, 130, 17, 0), (111, 97, 23, 1), (510, 254, 20, 0), (1022, 1020, 11, 0), (1445, 1441, 10, 1),
+])
+def test_noalloc_pass_edges(rt, dtype, nx, ny, sweeps, shift):
+    torch = pytest.importorskip("torch")
+    from charming_b200 import _lib
+    npdt = np.float64 if dtype == "f64" else np.float32
+    n = (nx + 2) * (ny + 2)
+    g = np.random.default_rng(nx * 7 + ny).random((ny + 2, nx + 2)).astype(npdt)
+    tdt = torch.float64 if dtype == "f64" else torch.float32
+    d_in = torch.empty(n + 4, dtype=tdt, device="cuda")
+    d_out = torch.full((n + 4,), float("nan"), dtype=tdt, device="cuda")
+    d_in[shift:shift + n] = torch.from_numpy(g.reshape(-1)).cuda()
+    esz = g.itemsize
+    _lib.check(rt.lib.charming_jacobi2d_sweeps_noalloc(_lib.F64 if dtype == "f64" else _lib.F32, nx, ny, sweeps,
+                                                       d_in.data_ptr() + shift * esz, d_out.data_ptr() + shift * esz))
+    out = d_out.cpu().numpy()
+    assert same_bits(out[shift:shift + n].reshape(g.shape).copy(), oracle(g, sweeps))
+    assert np.isnan(out[:shift]).all() and np.isnan(out[shift + n:]).all()  # nothing beyond the grid is written
+    assert same_bits(d_in[shift:shift + n].cpu().numpy().reshape(g.shape), g)
