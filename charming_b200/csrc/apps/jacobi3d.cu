@@ -9,253 +9,249 @@
 // sweeps alternate between two buffers, so the result is `sweeps` Jacobi
 // iterations.
 //
-// Two kernels, the same arithmetic. Each block owns a 32 x 16 tile of (x, y)
-// columns and a run of z planes and marches up z.
-//   jacobi3d_async_kernel (grids of at least one 34 x 18 box in x and y):
-//     the tile's planes, rim included, stream through a ring of J3_S
-//     shared-memory slots by per-thread asynchronous copies (cp.async, one
-//     commit group per plane), J3_S - 2 planes ahead of the one computed
-//     (J3_S = 10 by default; 256 threads, two tile rows each).
-//     Each input value is read from DRAM once per sweep (16 B per lattice
-//     update with the store); the rim cells come from L2.
-//   jacobi3d_kernel (any shape): per-thread loads, the planes below and
-//     above a thread's cell and one more in registers, the current plane
-//     with its rim in shared memory.
+// One kernel, L sweeps per pass over the grid (3 or 2; 1 for an odd last
+// sweep): a block owns a strip of 32 vectors of 2 columns times the rows of
+// its warps (RY each) and marches up z, one plane per step. A thread keeps,
+// per level and row, the newest plane of the level below (X) and the partial
+// sums of the first six terms around it (P, taken when that plane arrived);
+// the next plane closes them, (P + zp) * 0.142857, the adds in the same
+// order. So a plane's way through all levels needs no neighbours, and one
+// block barrier per plane (the rows at the warps' edges go through shared
+// memory, columns by shuffle) serves every level. The planes stream through a
+// private ring of shared-memory slots per thread (cp.async). Tiles overlap by
+// L cells on each side; the boundary shell is kept at every level and copied.
+// Bound by the load/store pipe (ring copies, edge rows, shuffles) and, on
+// small grids, by the chain of a plane's step. GLUP/s against one sweep per
+// pass (32 x 16 tiles, planes by cp.async): 256^3 399 (255), 512^3 507 (290),
+// 640^3 580 (293), 128^3 220, 299 x 300 x 250 428 (232).
 #include "suite.cuh"
 #ifndef CHARMING_HOST_EMULATION
 #include "jacobi_sweep.cuh"
 #include "../host.cuh"
+#include <algorithm>
 #include <cmath>
-#include <cstdlib>
 
 namespace {
 
-constexpr int J3_TX = 32, J3_TY = 16;
-constexpr int J3_BW = J3_TX + 2, J3_BH = J3_TY + 2;          // tensor box: tile + rim
-// 10 slots and 2 tile rows per thread: 293 GLUP/s at 640^3, against 265
-// with 8 slots and one row, 282 with 12 slots and two rows
-constexpr int J3_S_DEFAULT = 10;                             // plane slots
-constexpr int J3_RPT_DEFAULT = 2;                            // tile rows per thread
+constexpr int J3_S = 4;       // planes in the ring
+constexpr int J3_NWMAX = 16;  // warps per block
 
-__device__ __forceinline__ double j3_stencil(double c, double xm, double xp, double ym, double yp, double zm,
-    double zp) {
-  return __dmul_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(c, xm), xp), ym), yp), zm), zp),
-                   0.142857);
-}
+template <int L>
+struct j3_geom {
+  static constexpr int E = (L + 1) / 2;      // vectors lost at each strip edge
+  static constexpr int SS = 32 - 2 * E;      // vectors a strip owns
+};
+// rings of J3_S planes (RY rows per warp), and the edge rows of each warp,
+// level and step parity
+constexpr size_t j3_smem(int warps, int L, int RY) { return (size_t)warps * 512 * (J3_S * RY + 4 * L); }
 
-// Planes z0-1 .. z1 of the tile stream through J3_S shared-memory slots:
-// plane p lives in slot (p - z0 + 1) % J3_S, one cp.async group per plane
-// (8-byte copies of the 34 x 18 box: the tile and its rim; cells outside the
-// grid are zero-filled and never used). Before output plane z is computed,
-// planes up to z + J3_S - 2 are issued and wait_group leaves J3_S - 3 of
-// them in flight, so planes z-1, z, z+1 have landed. The block has
-// 32 x (16 / RPT) threads; each computes RPT rows of the tile.
-template <int J3_S, int RPT>
-__global__ void __launch_bounds__(J3_TX * J3_TY / RPT, 3 * RPT) jacobi3d_async_kernel(
-    const double* __restrict__ in, double* __restrict__ out, int nx, int ny, int nz, int zrun) {
-  extern __shared__ __align__(16) double j3_slots[];  // [J3_S][J3_BH][J3_BW]
-  constexpr int TY = J3_TY / RPT, NT = J3_TX * TY;
-  constexpr int BOX = J3_BW * J3_BH, SLOT = BOX;  // doubles per slot
-  constexpr int NC = (BOX + NT - 1) / NT;         // box cells per thread
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * J3_TX + tx;
-  const int bx0 = blockIdx.x * J3_TX, by0 = blockIdx.y * J3_TY;
-  const int x = bx0 + tx + 1;
-  const int z0 = 1 + blockIdx.z * zrun, z1 = min(nz + 1, z0 + zrun);
-  const long long sy = nx + 2, sz = (long long)(nx + 2) * (ny + 2);
-  int cell[NC], goff[NC];
-  bool inside[NC];
+struct j3_plan {
+  int warps, yown, yblocks, zrun, zruns, strips;
+  double cost;
+};
+
+template <int L, int RY, bool FIX>
+__device__ __forceinline__ void j3_tile(const double* __restrict__ in, double* __restrict__ out, int nx, int ny,
+    int nz, int pitch, int zrun, int yown, double2* smem) {
+  using G = j3_geom<L>;
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
+  const int NT = (int)blockDim.x, W = nx + 2;
+  const size_t plane = (size_t)pitch * (ny + 2);
+  const int own0 = (int)blockIdx.x * G::SS, col0 = (own0 - G::E + lane) * 2;
+  const int nv = (W + 1) / 2;
+  const bool own = lane >= G::E && lane < G::E + min(G::SS, nv - own0);
+  const int y0 = (int)blockIdx.y * yown, yt = y0 - L + warp * RY;  // the warp's first row
+  const int z0 = (int)blockIdx.z * zrun, z1 = min(nz + 2, z0 + zrun);
+  const int qs = z0 - L, qe = z1 - 1 + L;
+  const bool fixc0 = col0 == 0 || col0 == nx + 1, fixc1 = col0 + 1 == nx + 1;
+  // this thread's ring slots and the exchange rows
+  double2* ring = smem + threadIdx.x;
+  double2* ex = smem + (size_t)J3_S * RY * NT;  // [parity][level][first, last][thread]
+  // columns and rows off the grid: its nearest ones, never used by a result
+  long long goff[RY];
+  int nput[RY];
+  bool rowfix[RY];
+  const int c0 = min(max(col0, 0), pitch - 2);
 #pragma unroll
-  for (int k = 0; k < NC; k++) {
-    const int e = tid + k * NT;
-    cell[k] = e < BOX ? e : -1;
-    const int gx = bx0 + e % J3_BW, gy = by0 + e / J3_BW;
-    inside[k] = e < BOX && gx <= nx + 1 && gy <= ny + 1;
-    goff[k] = inside[k] ? (int)(gy * sy + gx) : 0;
+  for (int i = 0; i < RY; i++) {
+    const int y = yt + i;
+    goff[i] = (long long)min(max(y, 0), ny + 1) * pitch + c0;
+    rowfix[i] = y == 0 || y == ny + 1;
+    nput[i] = own && y >= y0 && y < min(y0 + yown, ny + 2) ? W - col0 : 0;
   }
-  auto issue = [&](int p) {
-    if (p <= z1) {
-      double* slot = j3_slots + ((p - z0 + 1) % J3_S) * SLOT;
-      const double* src = in + (long long)p * sz;
+  int next = qs;
+  auto fetch = [&](int slot) {
+    const double* src = in + (size_t)min(max(next, 0), nz + 1) * plane;
+    next++;
 #pragma unroll
-      for (int k = 0; k < NC; k++) {
-        if (cell[k] < 0) continue;
-        // zero-fill (source size 0) outside the grid, from a valid address
-        const unsigned n = inside[k] ? 8u : 0u;
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(jac::smem_u32(slot + cell[k])),
-                     "l"(inside[k] ? src + goff[k] : in), "r"(n) : "memory");
-      }
+    for (int i = 0; i < RY; i++) {
+      const unsigned dst = jac::smem_u32(ring + (slot * RY + i) * NT);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + goff[i]) : "memory");
     }
-    jac::cp_async_commit();  // one group per plane, empty past z1
+    jac::cp_async_commit();
   };
-  for (int p = z0 - 1; p <= z0 + J3_S - 3; p++) issue(p);
-  for (int z = z0; z < z1; z++) {
-    issue(z + J3_S - 2);              // into the slot plane z-2 used
-    jac::cp_async_wait<J3_S - 3>();  // planes up to z+1 have landed (this thread's copies)
-    __syncthreads();                 // ... and every other thread's
-    const double* m = j3_slots + ((z - z0 + 1) % J3_S) * SLOT;
-    const double* lo = j3_slots + ((z - z0) % J3_S) * SLOT;
-    const double* hi = j3_slots + ((z - z0 + 2) % J3_S) * SLOT;
+  for (int k = 0; k < J3_S - 1; k++) fetch(k);
+  double2 P[L][RY], X[L][RY];
 #pragma unroll
-    for (int r = 0; r < RPT; r++) {
-      const int yy = ty + r * TY, y = by0 + yy + 1;
-      if (x <= nx && y <= ny) {
-        const int c = (yy + 1) * J3_BW + tx + 1;
-        out[(long long)y * sy + x + (long long)z * sz] =
-            j3_stencil(m[c], m[c - 1], m[c + 1], m[c - J3_BW], m[c + J3_BW], lo[c], hi[c]);
+  for (int l = 0; l < L; l++)
+#pragma unroll
+    for (int i = 0; i < RY; i++) P[l][i] = X[l][i] = make_double2(0.0, 0.0);
+  int slot = 0, par = 0;
+  double* oplane = out + col0;
+#pragma unroll 1
+  for (int q = qs; q <= qe; q++) {
+    double2 v[L + 1][RY];
+    jac::cp_async_wait<J3_S - 2>();
+#pragma unroll
+    for (int i = 0; i < RY; i++) v[0][i] = ring[(slot * RY + i) * NT];
+    fetch(slot == 0 ? J3_S - 1 : slot - 1);  // the slot of the plane read before
+    slot = slot + 1 == J3_S ? 0 : slot + 1;
+    double2* e = ex + (size_t)par * L * 2 * NT + threadIdx.x;
+    par ^= 1;
+#pragma unroll
+    for (int l = 0; l < L; l++) {
+      e[(2 * l) * NT] = v[l][0];
+      e[(2 * l + 1) * NT] = v[l][RY - 1];
+      const int z = q - l - 1;  // plane of level l + 1 computed now
+      const bool zfix = FIX && (z == 0 || z == nz + 1);
+#pragma unroll
+      for (int i = 0; i < RY; i++) {
+        double2 o;
+        o.x = __dmul_rn(__dadd_rn(P[l][i].x, v[l][i].x), 0.142857);
+        o.y = __dmul_rn(__dadd_rn(P[l][i].y, v[l][i].y), 0.142857);
+        if (FIX) {
+          o.x = zfix || rowfix[i] || fixc0 ? X[l][i].x : o.x;
+          o.y = zfix || rowfix[i] || fixc1 ? X[l][i].y : o.y;
+        }
+        v[l + 1][i] = o;
       }
     }
-    __syncthreads();  // plane z-1's slot takes plane z+J3_S-1 next
+    const bool full = q >= qs + 2 * L;  // plane q - L is complete
+#pragma unroll
+    for (int i = 0; i < RY; i++) {
+      const int n = full ? nput[i] : 0;
+      double* p = oplane + (long long)(q - L) * (long long)plane + (yt + i) * (long long)pitch;
+      const double t[2] = {v[L][i].x, v[L][i].y};
+      jac::put_vec(p, t, n);
+    }
+    __syncthreads();  // the edge rows of every warp and level are there
+#pragma unroll
+    for (int l = 0; l < L; l++) {
+      // the rows above and below the warp's (at the block's edge: its own,
+      // never used by a result)
+      const double2 up = e[(2 * l + 1) * NT - (warp > 0 ? 32 : 0)];
+      const double2 dn = e[(2 * l) * NT + (warp + 1 < nw ? 32 : 0)];
+#pragma unroll
+      for (int i = 0; i < RY; i++) {
+        const double2 c = v[l][i];
+        const double left = __shfl_up_sync(FULL, c.y, 1), right = __shfl_down_sync(FULL, c.x, 1);
+        const double2 ym = i == 0 ? up : v[l][i - 1], yp = i == RY - 1 ? dn : v[l][i + 1];
+        P[l][i].x = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(c.x, left), c.y), ym.x), yp.x), X[l][i].x);
+        P[l][i].y = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(c.y, c.x), right), ym.y), yp.y), X[l][i].y);
+      }
+#pragma unroll
+      for (int i = 0; i < RY; i++) X[l][i] = v[l][i];
+    }
   }
   jac::cp_async_wait<0>();
 }
 
-__global__ void __launch_bounds__(J3_TX * J3_TY) jacobi3d_kernel(const double* __restrict__ in,
-    double* __restrict__ out, int nx, int ny, int nz, int zrun) {
-  __shared__ double plane[J3_TY + 2][J3_TX + 2];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int x = blockIdx.x * J3_TX + tx + 1, y = blockIdx.y * J3_TY + ty + 1;
-  const int z0 = 1 + blockIdx.z * zrun, z1 = min(nz + 1, z0 + zrun);
-  const long long sx = 1, sy = nx + 2, sz = (long long)(nx + 2) * (ny + 2);
-  const bool inx = x <= nx + 1, iny = y <= ny + 1;       // a cell of the grid (rim included)
-  const bool own = x <= nx && y <= ny;                   // an interior column
-  const long long col = (long long)(inx ? x : nx + 1) * sx + (long long)(iny ? y : ny + 1) * sy;
-  auto at = [&](int z) { return in[col + (long long)z * sz]; };
-  double prev = at(z0 - 1), cur = at(z0), next = at(z0 + 1);
-  for (int z = z0; z < z1; z++) {
-    const double nn = z + 2 <= nz + 1 ? at(z + 2) : 0.0;  // one plane ahead
-    plane[ty + 1][tx + 1] = cur;
-    const long long zo = (long long)z * sz;
-    if (tx == 0) plane[ty + 1][0] = in[col - sx + zo];
-    if (tx == J3_TX - 1 && inx && x + 1 <= nx + 1) plane[ty + 1][J3_TX + 1] = in[col + sx + zo];
-    if (ty == 0) plane[0][tx + 1] = in[col - sy + zo];
-    if (ty == J3_TY - 1 && iny && y + 1 <= ny + 1) plane[J3_TY + 1][tx + 1] = in[col + sy + zo];
-    __syncthreads();
-    if (own) {
-      out[col + zo] = j3_stencil(cur, plane[ty + 1][tx], plane[ty + 1][tx + 2], plane[ty][tx + 1],
-                                 plane[ty + 2][tx + 1], prev, next);
-    }
-    __syncthreads();
-    prev = cur;
-    cur = next;
-    next = nn;
-  }
+template <int L, int RY>
+__global__ void __launch_bounds__(32 * J3_NWMAX, 1) jacobi3d_pass_kernel(const double* __restrict__ in,
+    double* __restrict__ out, int nx, int ny, int nz, int pitch, int zrun, int yown) {
+  extern __shared__ __align__(16) double2 j3_shared[];
+  using G = j3_geom<L>;
+  const int own0 = (int)blockIdx.x * G::SS, y0 = (int)blockIdx.y * yown, z0 = (int)blockIdx.z * zrun;
+  // the tile's levels can meet the shell
+  const bool edge = own0 - G::E <= 0 || (own0 + G::SS + G::E) * 2 > nx + 1 || y0 - L <= 0 ||
+                    y0 - L + (int)(blockDim.x >> 5) * RY > ny + 1 || z0 - L <= 0 || z0 + zrun + L > nz + 1;
+  if (edge) j3_tile<L, RY, true>(in, out, nx, ny, nz, pitch, zrun, yown, j3_shared);
+  else j3_tile<L, RY, false>(in, out, nx, ny, nz, pitch, zrun, yown, j3_shared);
 }
 
-// The shared-memory pipeline needs no alignment beyond 8 bytes: any shape
-// with at least one full box in x and y takes it.
-bool async_shape_ok(int nx, int ny) { return nx + 2 >= J3_BW && ny + 2 >= J3_BH; }
-
-constexpr size_t j3_async_smem(int stages) { return (size_t)stages * J3_BW * J3_BH * 8; }
-
-// z planes per block for the register kernel: enough blocks to fill the GPU
-// several times over
-int jacobi3d_zrun(int nx, int ny, int nz, int n_sms) {
-  const long long cols = (long long)((nx + J3_TX - 1) / J3_TX) * ((ny + J3_TY - 1) / J3_TY);
-  long long want = 8LL * n_sms;  // blocks
-  long long runs = (want + cols - 1) / cols;
-  if (runs < 1) runs = 1;
-  int zrun = (int)((nz + runs - 1) / runs);
-  if (zrun < 16) zrun = 16;
-  return zrun;
-}
-
-// z planes per block for the pipelined kernel. Blocks = tiles x runs; the
-// GPU holds `slots` of them at once, so the launch takes ceil(blocks /
-// slots) waves and the last one may run part-empty, while every run reads
-// two planes more than it writes. Picks the run count (1..32) with the best
-// product of wave fill and plane efficiency.
-int jacobi3d_async_zrun(int nx, int ny, int nz, int n_sms, int per_sm) {
-  const long long tiles = (long long)((nx + J3_TX - 1) / J3_TX) * ((ny + J3_TY - 1) / J3_TY);
-  const double slots = (double)n_sms * (per_sm > 0 ? per_sm : 1);
-  int best_zrun = nz;
-  double best = -1.0;
-  for (int runs = 1; runs <= 32; runs++) {
-    const int zrun = (nz + runs - 1) / runs;
-    if (zrun < 8 && runs > 1) break;
-    const long long blocks = tiles * ((nz + zrun - 1) / zrun);
-    const double waves = (double)blocks / slots;
-    const double fill = waves / std::ceil(waves);
-    const double eff = fill * zrun / (zrun + 2.0);
-    if (eff > best + 1e-9) {
-      best = eff;
-      best_zrun = zrun;
+// Warps per block, rows per block and planes per run: the fewest steps of
+// all resident warps, over the waves that the launch takes. A block's rows
+// are its warps' less the 2L of the overlap, a run streams 2L planes more
+// than it writes; with few blocks the warps of an SM are bound by latency
+// (taken as 8 warps' worth of time).
+template <int L, int RY>
+j3_plan j3_choose(int nx, int ny, int nz, int n_sms) {
+  const int strips = ((nx + 2 + 1) / 2 + j3_geom<L>::SS - 1) / j3_geom<L>::SS;
+  j3_plan best{};
+  best.cost = 1e300;
+  for (int nw = (2 * L + RY) / RY; nw <= J3_NWMAX; nw++) {
+    const int ymax = nw * RY - 2 * L;
+    if (ymax < 1) continue;
+    const int yb = (ny + 2 + ymax - 1) / ymax;
+    if (yb > 65535 && nw < J3_NWMAX) continue;  // grid limit
+    const int yown = (ny + 2 + yb - 1) / yb;
+    const int per_sm = std::max(1, std::min(J3_NWMAX / nw, (int)((227u << 10) / (j3_smem(nw, L, RY) + 1024))));
+    const long long tiles = (long long)strips * yb;
+    for (int runs = 1; runs <= 64; runs++) {
+      const int zr = (nz + 2 + runs - 1) / runs;
+      if (runs > 1 && zr < 4 * L) break;
+      const long long blocks = tiles * ((nz + 2 + zr - 1) / zr);
+      const double waves = std::ceil((double)blocks / ((double)n_sms * per_sm));
+      const double resident = std::min<double>(per_sm, std::ceil((double)blocks / n_sms));
+      const double cost = waves * (zr + 2 * L) * std::max(8.0, resident * nw) * RY / L;
+      if (cost < best.cost * 0.999) best = j3_plan{nw, yown, yb, zr, (nz + 2 + zr - 1) / zr, strips, cost};
+      if (zr == 1) break;
     }
   }
-  return best_zrun;
+  return best;
 }
 
-// Rows per thread of the pipelined kernel: CHARMING_J3_RPT (1 or 2) with
-// CHARMING_J3_STAGES (8 with 1 row, 10 or 12 with 2), else the defaults.
-int jacobi3d_rpt() {
-  static int rpt = 0;
-  if (!rpt) {
-    rpt = J3_RPT_DEFAULT;
-    if (const char* ev = getenv("CHARMING_J3_RPT")) {
-      const int v = atoi(ev);
-      if (v == 1 || v == 2) rpt = v;
-    }
-  }
-  return rpt;
-}
-
-// Stage count of the pipelined kernel (see jacobi3d_rpt).
-int jacobi3d_stages() {
-  static int stages = 0;
-  if (!stages) {
-    stages = J3_S_DEFAULT;
-    if (const char* ev = getenv("CHARMING_J3_STAGES")) {
-      const int v = atoi(ev);
-      if (v == 8 || v == 10 || v == 12) stages = v;
-    }
-  }
-  return stages;
-}
-
-template <int S, int RPT>
-cudaError_t jacobi3d_async_sweeps(double*& a, double*& b, int nx, int ny, int nz, int sweeps, int n_sms,
+template <int L, int RY>
+cudaError_t j3_pass(const double* in, double* out, int nx, int ny, int nz, int pitch, const j3_plan& p,
     cudaStream_t s) {
-  int per_sm = 0;
-  cudaError_t e = cudaSuccess;
-  const void* fn = (const void*)jacobi3d_async_kernel<S, RPT>;
-  if (j3_async_smem(S) > 48 * 1024)
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)j3_async_smem(S));
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, jacobi3d_async_kernel<S, RPT>,
-                                                      J3_TX * J3_TY / RPT, j3_async_smem(S));
+  auto fn = jacobi3d_pass_kernel<L, RY>;
+  const size_t smem = j3_smem(p.warps, L, RY);
+  cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)j3_smem(J3_NWMAX, L, RY));
   if (e != cudaSuccess) return e;
-  const int zrun = jacobi3d_async_zrun(nx, ny, nz, n_sms, per_sm);
-  const dim3 block(J3_TX, J3_TY / RPT), grid((nx + J3_TX - 1) / J3_TX, (ny + J3_TY - 1) / J3_TY, (nz + zrun - 1) / zrun);
-  for (int k = 0; k < sweeps && e == cudaSuccess; k++) {
-    jacobi3d_async_kernel<S, RPT><<<grid, block, j3_async_smem(S), s>>>(a, b, nx, ny, nz, zrun);
-    e = cudaGetLastError();
-    double* t = a;
-    a = b;
-    b = t;
-  }
-  return e;
+  fn<<<dim3(p.strips, p.yblocks, p.zruns), 32 * p.warps, smem, s>>>(in, out, nx, ny, nz, pitch, p.zrun, p.yown);
+  return cudaGetLastError();
 }
 
-// `sweeps` sweeps alternating between a and b (both hold the input,
-// boundary shell included); returns the buffer holding the result.
-double* jacobi3d_run(double* a, double* b, int nx, int ny, int nz, int sweeps, cudaStream_t s, cudaError_t* err) {
+// Rows of an odd number of columns are kept in rows one double longer, so that
+// every row starts on a 16-byte boundary (element copies and stores made the
+// sweeps of a 255^3 grid 1.65 times as long); these copy them between.
+__global__ void __launch_bounds__(256) j3_repitch_kernel(const double* __restrict__ src, double* __restrict__ dst,
+    int W, int sp, int dp, long long rows) {
+  for (long long r = (long long)blockIdx.x; r < rows; r += (long long)gridDim.x)
+    for (int c = (int)threadIdx.x; c < W; c += 256) dst[r * dp + c] = src[r * sp + c];
+}
+cudaError_t j3_repitch(const double* src, double* dst, int W, int sp, int dp, long long rows,
+    cudaStream_t s) {
+  j3_repitch_kernel<<<(unsigned)std::min<long long>(rows, 148 * 16), 256, 0, s>>>(src, dst, W, sp, dp, rows);
+  return cudaGetLastError();
+}
+
+// `sweeps` sweeps from a, alternating between a and b (a pass writes its whole
+// target, shell included); returns the buffer holding the result.
+double* jacobi3d_run(double* a, double* b, int nx, int ny, int nz, int pitch, int sweeps, cudaStream_t s,
+    cudaError_t* err) {
   const int n_sms = charm_host::info().n_sms;
   *err = cudaSuccess;
-  const dim3 block(J3_TX, J3_TY);
-  if (async_shape_ok(nx, ny)) {
-    const int st = jacobi3d_stages(), rpt = jacobi3d_rpt();
-    if (st == 8 && rpt == 1) *err = jacobi3d_async_sweeps<8, 1>(a, b, nx, ny, nz, sweeps, n_sms, s);
-    else if (st == 12 && rpt == 2) *err = jacobi3d_async_sweeps<12, 2>(a, b, nx, ny, nz, sweeps, n_sms, s);
-    else *err = jacobi3d_async_sweeps<10, 2>(a, b, nx, ny, nz, sweeps, n_sms, s);
-    return a;
-  }
-  const int zrun = jacobi3d_zrun(nx, ny, nz, n_sms);
-  const dim3 grid((nx + J3_TX - 1) / J3_TX, (ny + J3_TY - 1) / J3_TY, (nz + zrun - 1) / zrun);
-  for (int k = 0; k < sweeps && *err == cudaSuccess; k++) {
-    jacobi3d_kernel<<<grid, block, 0, s>>>(a, b, nx, ny, nz, zrun);
-    *err = cudaGetLastError();
-    double* t = a;
-    a = b;
-    b = t;
+  const j3_plan p3 = j3_choose<3, 2>(nx, ny, nz, n_sms), p2 = j3_choose<2, 3>(nx, ny, nz, n_sms),
+                p1 = j3_choose<1, 3>(nx, ny, nz, n_sms);
+  // Three sweeps per pass take fewer plane steps but overlap by more rows, and
+  // one of their row steps costs 1.1 to 1.26 of the other's. 256^3: 42 us per
+  // sweep against 47 with two, 128^3 9.5 against 12.3; 512^3 276 against 265.
+  const bool three = p3.cost * 1.24 < p2.cost;
+  while (sweeps > 0 && *err == cudaSuccess) {
+    if (three && sweeps >= 3) {
+      *err = j3_pass<3, 2>(a, b, nx, ny, nz, pitch, p3, s);
+      sweeps -= 3;
+    } else if (sweeps >= 2) {
+      *err = j3_pass<2, 3>(a, b, nx, ny, nz, pitch, p2, s);
+      sweeps -= 2;
+    } else {
+      *err = j3_pass<1, 3>(a, b, nx, ny, nz, pitch, p1, s);
+      sweeps--;
+    }
+    std::swap(a, b);
   }
   return a;
 }
@@ -267,20 +263,27 @@ extern "C" int charming_jacobi3d(int nx, int ny, int nz, int sweeps, double* gri
   if (rc) return rc;
   if (nx < 1 || ny < 1 || nz < 1 || sweeps < 0 || !grid) return CHARMING_ERR_CONFIG;
   const size_t n = ((size_t)nx + 2) * ((size_t)ny + 2) * ((size_t)nz + 2);
+  // device rows start on 16-byte boundaries; a grid of odd rows passes through
+  // b on its way in and through the other buffer on its way out
+  const int W = nx + 2, pitch = W + (W & 1);
+  const long long rows = ((long long)ny + 2) * ((long long)nz + 2);
+  const size_t np = (size_t)pitch * (size_t)rows;
   double *a = nullptr, *b = nullptr;
-  cudaError_t e = cudaMalloc(&a, n * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&b, n * 8);
+  cudaError_t e = cudaMalloc(&a, np * 8);
+  if (e == cudaSuccess) e = cudaMalloc(&b, np * 8);
   cudaStream_t s = charm_host::stream();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(a, grid, n * 8, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(b, a, n * 8, cudaMemcpyDeviceToDevice, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(pitch == W ? a : b, grid, n * 8, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && pitch != W) e = j3_repitch(b, a, W, W, pitch, rows, s);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (e == cudaSuccess) e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
   double* res = a;
   if (e == cudaSuccess) e = cudaEventRecord(e0, s);
-  if (e == cudaSuccess) res = jacobi3d_run(a, b, nx, ny, nz, sweeps, s, &e);
+  if (e == cudaSuccess) res = jacobi3d_run(a, b, nx, ny, nz, pitch, sweeps, s, &e);
   if (e == cudaSuccess) e = cudaEventRecord(e1, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(grid, res, n * 8, cudaMemcpyDeviceToHost, s);
+  double* flat = pitch == W ? res : res == a ? b : a;
+  if (e == cudaSuccess && pitch != W) e = j3_repitch(res, flat, W, pitch, W, rows, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(grid, flat, n * 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   float ms = 0.f;
   if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);

@@ -101,3 +101,16 @@ def test_noalloc_pass_edges(rt, dtype, nx, ny, sweeps, shift):
     assert same_bits(out[shift:shift + n].reshape(g.shape).copy(), oracle(g, sweeps))
     assert np.isnan(out[:shift]).all() and np.isnan(out[shift + n:]).all()  # nothing beyond the grid is written
     assert same_bits(d_in[shift:shift + n].cpu().numpy().reshape(g.shape), g)
+
+
+# charming_jacobi3d: grids smaller than a warp's strip and rows, strip (60
+# columns for two sweeps, 62 for one) and row remainders, odd widths (element
+# copies), runs of planes, odd sweep counts (a last pass of one sweep)
+@pytest.mark.parametrize("nx,ny,nz,sweeps", [
+    (1, 1, 1, 3), (3, 2, 5, 4), (58, 44, 9, 2), (59, 45, 10, 3), (61, 46, 33, 1), (62, 5, 70, 6), (120, 100, 40, 4),
+    (257, 31, 12, 5), (20, 300, 16, 2), (124, 90, 130, 7),
+])
+def test_jacobi3d_tile_edges(rt, nx, ny, nz, sweeps):
+    g = np.random.default_rng(nx + ny + nz).random((nz + 2, ny + 2, nx + 2))
+    out, _ms = rt.jacobi3d(g, sweeps)
+    assert same_bits(out, oj.jacobi3d(g, sweeps))
