@@ -43,7 +43,7 @@ constexpr int HDR = 32;                  // envelope (16) + regular_msg (16)
 constexpr int MAX_THREADS = CHARMING_MAX_THREADS;  // launch bound of the scheduler
 constexpr int PROXY_CACHE = 16;          // proxies per PE looked up on chip
 constexpr int SMEM_OBJ_MAX = 4096;       // larger objects skip the on-chip arena
-constexpr int RQ_MAX = 256;              // ready stash entries listed on chip
+constexpr int RQ_MAX = 128;              // ready stash entries listed on chip
 
 struct alignas(128) line_u64 {
   unsigned long long v;
@@ -62,6 +62,13 @@ struct stash_key {
 };
 
 enum : int { KEY_FREE = 0, KEY_WAIT = 1, KEY_READY = 2 };
+
+// A ready stashed message as the on-chip list keeps it.
+struct ready_rec {
+  int idx, refnum;
+  unsigned short cid, ep;
+  unsigned int off16;           // its offset in the PE's arena, in 16-byte units
+};
 
 // Outbox entry header, 32 B; the message (envelope, header, payload) follows.
 struct ob_entry {
@@ -227,8 +234,11 @@ struct pe_state {
   // ready stashed messages found by the last revive, in key order (offsets
   // from rq_base); rq_over: more than RQ_MAX, scan from ready_cursor instead
   unsigned long long rq_base;
+  // with what a delivery needs of each, read by the revive's threads together
+  // (rq: offset << 8 | record)
   int rq_n, rq_pos, rq_over;
   unsigned int rq[RQ_MAX];
+  ready_rec rq_rec[RQ_MAX];
   // block-collective broadcast slots
   void* b_ptr0;
   const void* b_ptr1;
@@ -267,6 +277,9 @@ struct pe_state {
   chare_proxy_base* bp[MAX_THREADS / 32];
   void* barg[MAX_THREADS / 32];
   int bidx[MAX_THREADS / 32], bep[MAX_THREADS / 32];
+  unsigned int b_early;                // members (bits) that are early messages, copied to the stash:
+  void* bdst[MAX_THREADS / 32];        // their arena addresses, from the messages at barg
+  unsigned int bbytes[MAX_THREADS / 32];
   unsigned long long bstash[MAX_THREADS / 32];  // stash keys of a stash batch
   unsigned long long bkeys[MAX_THREADS / 32];   // its chares
   // the block-shared message array of block_messages() (raw storage: the

@@ -1024,7 +1024,19 @@ __device__ void stash_revive_scan() {
     }
     if (st == KEY_READY) {
       const int pos = atomicAdd_block(&ps->rq_n, 1);
-      if (pos < RQ_MAX) ps->rq[pos] = (unsigned int)(i - kh);
+      const unsigned long long off = k->data_off % c_rt.stash_bytes;
+      if (pos < RQ_MAX && i - kh < (1ULL << 24) && off < (1ULL << 36)) {
+        const unsigned char* env = arena_of(blockIdx.x) + off;
+        ready_rec& q = ps->rq_rec[pos];
+        q.idx = k->chare_idx;
+        q.refnum = k->refnum;
+        q.cid = (unsigned short)k->chare_id;  // (both below their table sizes)
+        q.ep = (unsigned short)reinterpret_cast<const regular_msg*>(env + sizeof(envelope))->ep_id;
+        q.off16 = (unsigned int)(off >> 4);
+        ps->rq[pos] = (unsigned int)(i - kh) << 8 | (unsigned int)pos;
+      } else {
+        atomicExch_block(&ps->rq_over, 1);
+      }
     }
   }
   if (cnt) atomicAdd_block(&ps->red_i[0], cnt);
@@ -1033,10 +1045,7 @@ __device__ void stash_revive_scan() {
 // Thread 0: the ready list of the last revive in key (arrival) order.
 __device__ void ready_list_sort() {
   pe_state* ps = pes();
-  if (ps->rq_n > RQ_MAX) {
-    ps->rq_over = 1;
-    ps->rq_n = RQ_MAX;
-  }
+  if (ps->rq_over) return;  // not all are listed: the keys are scanned instead
   for (int a = 1; a < ps->rq_n; a++) {  // insertion sort: short lists
     const unsigned int v = ps->rq[a];
     int b = a - 1;
@@ -1050,19 +1059,21 @@ __device__ void ready_list_sort() {
 }
 
 // Thread 0: the oldest ready stashed message, or ~0 when none is left:
-// from the ready list, or, when that overflowed, by scanning the keys
-// from ready_cursor (keys before it are known not to be ready).
-__device__ unsigned long long stash_next_ready() {
+// from the ready list (*rec: its record there), or, when that overflowed, by
+// scanning the keys from ready_cursor (keys before it are known not to be
+// ready; *rec -1). A listed message stays ready until its delivery takes it
+// off the list, or until next_action puts it back to waiting.
+__device__ unsigned long long stash_next_ready(int* rec) {
   pe_state* ps = pes();
   const unsigned long long S = (unsigned long long)c_rt.stash_entries;
   stash_key* keys = keys_of(blockIdx.x);
   if (!ps->rq_over) {
-    while (ps->rq_pos < ps->rq_n) {
-      const unsigned long long i = ps->rq_base + ps->rq[ps->rq_pos++];
-      if (i >= ps->key_head && i < ps->key_tail && keys[i % S].state == KEY_READY) return i;
-    }
-    return ~0ULL;
+    if (ps->rq_pos >= ps->rq_n) return ~0ULL;
+    const unsigned int q = ps->rq[ps->rq_pos++];
+    *rec = (int)(q & 255);
+    return ps->rq_base + (q >> 8);
   }
+  *rec = -1;
   unsigned long long i = ps->ready_cursor < ps->key_head ? ps->key_head : ps->ready_cursor;
   for (; i < ps->key_tail; i++)
     if (keys[i % S].state == KEY_READY) {
@@ -1256,8 +1267,9 @@ __device__ void finish_action() {
       ps->head += ps->nb_cells;
       if (ps->head - ps->head_pub >= (c_rt.ring_cells >> 3)) publish_head(ps, me);
       const unsigned long long d0 = ps->stats[ST_DELIVERED];
-      ps->stats[ST_DELIVERED] = d0 + (unsigned long long)ps->nb;
-      if (ps->nb > 1) ps->stats[ST_BATCHED] += (unsigned long long)ps->nb;
+      const int calls = ps->nb - __popc(ps->b_early);
+      ps->stats[ST_DELIVERED] = d0 + (unsigned long long)calls;
+      if (calls > 1) ps->stats[ST_BATCHED] += (unsigned long long)calls;
       if ((d0 >> 4) != (ps->stats[ST_DELIVERED] >> 4)) stamp_progress(me);
       break;
     }
@@ -1287,42 +1299,37 @@ __device__ void finish_action() {
 // while each is for a warp-level entry method of a chare not yet in the
 // batch and its refnum matches (the first that is not is left for the
 // next decision, as for inbox batches).
-__device__ void stash_batch(chare_proxy_base* p, const stash_key* k, int ep, void* arg, unsigned long long i) {
+__device__ void stash_batch(chare_proxy_base* p, int cid, int idx, int ep, void* arg, unsigned long long i) {
   pe_state* ps = pes();
-  const unsigned long long S = (unsigned long long)c_rt.stash_entries;
-  stash_key* keys = keys_of(blockIdx.x);
   const int maxb = (int)(blockDim.x >> 5);
   ps->d_act = ACT_STASH_BATCH;
   ps->nb = 1;
   ps->bp[0] = p;
-  ps->bidx[0] = k->chare_idx;
+  ps->bidx[0] = idx;
   ps->bep[0] = ep;
   ps->barg[0] = arg;
   ps->bstash[0] = i;
-  ps->bkeys[0] = ((unsigned long long)(unsigned)k->chare_id << 32) | (unsigned)k->chare_idx;
+  ps->bkeys[0] = ((unsigned long long)(unsigned)cid << 32) | (unsigned)idx;
   while (ps->nb < maxb && ps->n_ready > ps->nb) {
     const int pos = ps->rq_pos;
-    const unsigned long long cur = ps->ready_cursor;
-    const unsigned long long j = stash_next_ready();
+    int rec = 0;
+    const unsigned long long j = stash_next_ready(&rec);  // (listed: rq_over takes no batch)
     bool take = j != ~0ULL;
-    const stash_key* kj = take ? keys + (j % S) : nullptr;
-    chare_proxy_base* pj = take ? proxy_of(ps, kj->chare_id) : nullptr;
-    const unsigned char* env = take ? arena_of(blockIdx.x) + (kj->data_off % c_rt.stash_bytes) : nullptr;
-    const int epj = take ? reinterpret_cast<const regular_msg*>(env + sizeof(envelope))->ep_id : 0;
-    const unsigned long long key =
-        take ? ((unsigned long long)(unsigned)kj->chare_id << 32) | (unsigned)kj->chare_idx : 0;
-    take = take && pj->warp_em(epj) && pj->refnum_matches(kj->chare_idx, kj->refnum);
+    const ready_rec q = ps->rq_rec[rec];
+    chare_proxy_base* pj = take ? proxy_of(ps, q.cid) : nullptr;
+    const int idxj = q.idx, epj = q.ep;
+    const unsigned long long key = ((unsigned long long)q.cid << 32) | (unsigned)idxj;
+    take = take && pj->warp_em(epj) && pj->refnum_matches(idxj, q.refnum);
     for (int b = 0; take && b < ps->nb; b++) take = ps->bkeys[b] != key;
     if (!take) {  // leave it for the next decision
       ps->rq_pos = pos;
-      ps->ready_cursor = cur;
       break;
     }
     const int n = ps->nb;
     ps->bp[n] = pj;
-    ps->bidx[n] = kj->chare_idx;
+    ps->bidx[n] = idxj;
     ps->bep[n] = epj;
-    ps->barg[n] = const_cast<unsigned char*>(env) + HDR;
+    ps->barg[n] = arena_of(blockIdx.x) + ((unsigned long long)q.off16 << 4) + HDR;
     ps->bstash[n] = j;
     ps->bkeys[n] = key;
     ps->nb = n + 1;
@@ -1395,14 +1402,18 @@ __device__ void next_action() {
     }
     // ready stashed messages go before new inbox messages, oldest first
     while (ps->n_ready > 0) {
-      const unsigned long long i = stash_next_ready();
+      int rec = 0;
+      const unsigned long long i = stash_next_ready(&rec);
       if (i == ~0ULL) {
         ps->n_ready = 0;
         break;
       }
       stash_key* k = keys_of(slot) + (i % S);
-      chare_proxy_base* p = proxy_of(ps, k->chare_id);
-      if (!p->refnum_matches(k->chare_idx, k->refnum)) {  // refnum moved on again
+      // from the list's record, on chip; with an overflowed list from the key
+      const ready_rec* q = rec >= 0 ? &ps->rq_rec[rec] : nullptr;
+      const int cid = q ? q->cid : k->chare_id, idx = q ? q->idx : k->chare_idx;
+      chare_proxy_base* p = proxy_of(ps, cid);
+      if (!p->refnum_matches(idx, q ? q->refnum : k->refnum)) {  // refnum moved on again
         k->state = KEY_WAIT;
         ps->n_ready--;
         ps->n_waiting++;
@@ -1412,10 +1423,9 @@ __device__ void next_action() {
         ps->d_act = ACT_EXIT;
         return;
       }
-      const unsigned char* env = arena_of(slot) + (k->data_off % c_rt.stash_bytes);
-      const regular_msg* rm = reinterpret_cast<const regular_msg*>(env + sizeof(envelope));
-      int ep = rm->ep_id;
-      if (inline_done(ps, p, k->chare_idx, &ep, const_cast<unsigned char*>(env) + HDR)) {
+      unsigned char* env = arena_of(slot) + (q ? (unsigned long long)q->off16 << 4 : k->data_off % c_rt.stash_bytes);
+      int ep = q ? q->ep : reinterpret_cast<const regular_msg*>(env + sizeof(envelope))->ep_id;
+      if (inline_done(ps, p, idx, &ep, env + HDR)) {
         k->state = KEY_FREE;
         ps->n_ready--;
         stash_retire();
@@ -1424,12 +1434,12 @@ __device__ void next_action() {
       }
       ps->d_act = ACT_CALL_STASH;
       ps->d_p = p;
-      ps->d_idx = k->chare_idx;
+      ps->d_idx = idx;
       ps->d_ep = ep;
-      ps->d_arg = const_cast<unsigned char*>(env) + HDR;
+      ps->d_arg = env + HDR;
       ps->d_key = i;
       // (from the on-chip ready list; past RQ_MAX ready ones, one at a time)
-      if (p->warp_em(rm->ep_id) && batching() && !ps->rq_over) stash_batch(p, k, rm->ep_id, ps->d_arg, i);
+      if (p->warp_em(ep) && batching() && q) stash_batch(p, cid, idx, ep, ps->d_arg, i);
       return;
     }
     if (ps->revive_pending) continue;
@@ -1463,27 +1473,38 @@ __device__ void next_action() {
         set_error(CHARMING_ERR_BAD_TARGET, cid, rm->chare_idx);
       } else if (p->refnum_matches(rm->chare_idx, rm->refnum)) {
         int ep = rm->ep_id;
-        if (!inline_done(ps, p, rm->chare_idx, &ep, m + HDR)) {
+        if (p->warp_em(ep) && batching()) {
+          // the first of a batch; warp 0 looks for more behind it
+          ps->d_act = ACT_CALL_BATCH;
+          ps->nb = 1;
+          ps->b_early = 0;
+          ps->nb_cells = cells_for(size);
+          ps->bkey0 = ((unsigned long long)(unsigned)cid << 32) | (unsigned)rm->chare_idx;
+          ps->bp[0] = p;
+          ps->bidx[0] = rm->chare_idx;
+          ps->bep[0] = ep;
+          ps->barg[0] = m + HDR;
+        } else if (!inline_done(ps, p, rm->chare_idx, &ep, m + HDR)) {
           ps->d_act = ACT_CALL_RING;
           ps->d_p = p;
           ps->d_idx = rm->chare_idx;
           ps->d_ep = ep;
           ps->d_arg = m + HDR;
         }
-        if (p->warp_em(rm->ep_id) && batching()) {
-          // the first of a batch; warp 0 looks for more behind it
-          ps->d_act = ACT_CALL_BATCH;
-          ps->nb = 1;
-          ps->nb_cells = cells_for(size);
-          ps->bkey0 = ((unsigned long long)(unsigned)cid << 32) | (unsigned)rm->chare_idx;
-          ps->bp[0] = p;
-          ps->bidx[0] = rm->chare_idx;
-          ps->bep[0] = rm->ep_id;
-          ps->barg[0] = m + HDR;
-        }
       } else {
         unsigned char* dst = stash_alloc(size, cid, rm->chare_idx, rm->refnum, env->src_pe);
-        if (dst) {
+        if (dst && batching() && p->warp_em(rm->ep_id)) {
+          // an early message for a warp-level entry method: one warp copies
+          // it, others take what follows it
+          ps->d_act = ACT_CALL_BATCH;
+          ps->nb = 1;
+          ps->b_early = 1;
+          ps->nb_cells = cells_for(size);
+          ps->bkey0 = ~0ULL;
+          ps->bdst[0] = dst;
+          ps->barg[0] = m;
+          ps->bbytes[0] = (unsigned int)size;
+        } else if (dst) {
           ps->d_act = ACT_STASH_PUT;
           ps->d_p = dst;
           ps->d_arg = m;
@@ -1510,9 +1531,12 @@ __device__ void next_action() {
 // published in the next 64 cells, and one more reads their envelopes.
 // Messages follow one another without gaps (each took its cells'
 // tickets), so the batch follows the chain from the first message's end
-// while each next message is published, is for a warp-level entry method
-// of a chare not yet in the batch, and its refnum matches; it stops at the
-// first that is not, which the scheduler then takes alone. The batch runs
+// while each next message is published and is for a warp-level entry method
+// of a chare without a delivery in the batch yet; it stops at the first
+// that is not, which the scheduler then takes alone. A member whose refnum
+// matches is a delivery; one that came early is copied to the stash by its
+// warp (with refnums three quarters of a fan-out's messages are early, and as
+// one block action each they were a third of its time). The batch runs
 // after a barrier, so the refnums checked here are the ones the sequential
 // order would check: an entry method of the batch changes only its own
 // chare's refnum.
@@ -1534,7 +1558,7 @@ __device__ __forceinline__ scan_cell scan_one(pe_state* ps, int me, unsigned lon
       chare_proxy_base* q = proxy_of(ps, rm->chare_id);
       c.idx = rm->chare_idx;
       c.ep = rm->ep_id;
-      c.ok = q && q->valid_target(c.idx, c.ep) && q->warp_em(c.ep) && q->refnum_matches(c.idx, rm->refnum);
+      if (q && q->valid_target(c.idx, c.ep) && q->warp_em(c.ep)) c.ok = q->refnum_matches(c.idx, rm->refnum) ? 1 : 2;
       c.cells = cells_for(size);
       c.key = ((unsigned long long)(unsigned)rm->chare_id << 32) | (unsigned)c.idx;
       c.p = reinterpret_cast<unsigned long long>(q);
@@ -1555,11 +1579,13 @@ __device__ void batch_extend() {
   // lane j holds the chare of batch member j
   unsigned long long mkey = lane == 0 ? ps->bkey0 : ~0ULL;
   int n = ps->nb, pos = 0;
+  unsigned int early = ps->b_early;
   unsigned int total = ps->nb_cells;
   while (n < maxb && pos < 64) {  // uniform: every lane computes the same
     const bool w0 = pos < 32;
     const int src = pos & 31;
-    if (!__shfl_sync(FULL, w0 ? lo.ok : hi.ok, src)) break;
+    const int kind = __shfl_sync(FULL, w0 ? lo.ok : hi.ok, src);
+    if (!kind) break;
     const unsigned long long k = __shfl_sync(FULL, w0 ? lo.key : hi.key, src);
     if (__any_sync(FULL, lane < n && mkey == k)) break;
     const unsigned int cl = __shfl_sync(FULL, w0 ? lo.cells : hi.cells, src);
@@ -1567,8 +1593,23 @@ __device__ void batch_extend() {
     const unsigned long long ba = __shfl_sync(FULL, w0 ? lo.arg : hi.arg, src);
     const int bi = __shfl_sync(FULL, w0 ? lo.idx : hi.idx, src);
     const int be = __shfl_sync(FULL, w0 ? lo.ep : hi.ep, src);
-    if (lane == n) mkey = k;
-    if (lane == 0) {
+    if (kind == 2) {  // its stash descriptor and arena space, by lane 0
+      unsigned long long dst = 0;
+      unsigned char* m = reinterpret_cast<unsigned char*>(ba) - HDR;
+      if (lane == 0) {
+        const envelope* env = reinterpret_cast<const envelope*>(m);
+        const regular_msg* rm = reinterpret_cast<const regular_msg*>(m + sizeof(envelope));
+        dst = reinterpret_cast<unsigned long long>(stash_alloc(env->size, rm->chare_id, bi, rm->refnum, env->src_pe));
+        ps->bdst[n] = reinterpret_cast<void*>(dst);
+        ps->barg[n] = m;
+        ps->bbytes[n] = (unsigned int)env->size;
+      }
+      if (!__shfl_sync(FULL, dst, 0)) break;  // stash full: error recorded
+      early |= 1u << n;
+    } else if (lane == n) {
+      mkey = k;
+    }
+    if (kind == 1 && lane == 0) {
       ps->bp[n] = reinterpret_cast<chare_proxy_base*>(bp);
       ps->barg[n] = reinterpret_cast<void*>(ba);
       ps->bidx[n] = bi;
@@ -1580,6 +1621,7 @@ __device__ void batch_extend() {
   }
   if (lane == 0) {
     ps->nb = n;
+    ps->b_early = early;
     ps->nb_cells = total;
   }
 }
@@ -1627,8 +1669,12 @@ __device__ void scheduler_loop() {
       }
       const int w = (int)(threadIdx.x >> 5);
       if (w < ps->nb) {
-        chare_proxy_base* q = ps->bp[w];
-        q->em_tab[ps->bep[w]](q, ps->bidx[w], ps->barg[w]);
+        if (act == ACT_CALL_BATCH && (ps->b_early >> w & 1u)) {
+          copy_cooperative(ps->bdst[w], ps->barg[w], ps->bbytes[w], threadIdx.x & 31, 32);
+        } else {
+          chare_proxy_base* q = ps->bp[w];
+          q->em_tab[ps->bep[w]](q, ps->bidx[w], ps->barg[w]);
+        }
       }
       if (threadIdx.x == 0) ps->stats[ST_EM_CYC] += (unsigned long long)(clock64() - c0);
     } else if (act == ACT_STASH_PUT) {
