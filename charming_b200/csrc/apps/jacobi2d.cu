@@ -178,6 +178,24 @@ __device__ int pass_len(const jac::chare_desc& d, const jac::prob_desc& p, int i
   return L < 1 ? 1 : L;
 }
 
+#if !defined(CHARMING_HOST_EMULATION) || defined(CHARMING_HOST_EMULATION_TMA)
+// The bulk-copy sweep with its plan (out of line, see send_packed; the plan
+// is made here, so that the sweep keeps it in registers). False: no plan for
+// this width.
+template <typename T, bool RESID>
+__device__ __noinline__ bool sweep_pipeline(const jac::chare_desc& d, jac::block_view<T> in, jac::block_view<T> out,
+    double* acc) {
+  size_t sb = 0;
+  void* sm = charm::smem_scratch(&sb);
+  jac::tma_plan P;
+  if (!jac::make_plan<T>(d.w, blockDim.x, sb, japp::tile_w(), &P)) return false;
+  double a = 0.0;
+  jac::sweep_tma<T, RESID>(in, out, d.w, d.h, sm, sb, P, &a);
+  *acc = a;
+  return true;
+}
+#endif
+
 // One pass of L sweeps buf[cur] -> buf[cur^1]; returns the block's residual
 // sum of the pass's first sweep (FP64, deterministic) when resid is set.
 // All threads.
@@ -202,16 +220,8 @@ __device__ double sweep_block(const jac::chare_desc& d, int cur, bool resid, int
     done = true;
   }
 #if !defined(CHARMING_HOST_EMULATION) || defined(CHARMING_HOST_EMULATION_TMA)
-  if (!done && japp::pipeline()) {
-    size_t sb = 0;
-    void* sm = charm::smem_scratch(&sb);
-    jac::tma_plan P;
-    if (jac::make_plan<T>(d.w, blockDim.x, sb, japp::tile_w(), &P)) {
-      if (resid) jac::sweep_tma<T, true>(in, out, d.w, d.h, sm, sb, P, &acc);
-      else jac::sweep_tma<T, false>(in, out, d.w, d.h, sm, sb, P, &acc);
-      done = true;
-    }
-  }
+  if (!done && japp::pipeline())
+    done = resid ? sweep_pipeline<T, true>(d, in, out, &acc) : sweep_pipeline<T, false>(d, in, out, &acc);
 #endif
   if (!done) {
     __syncthreads();

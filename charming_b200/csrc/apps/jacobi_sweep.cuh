@@ -844,7 +844,7 @@ __device__ bool make_plan(int w, int nthreads, size_t smem_bytes, int tile_w_opt
 // waiting, so it never blocks the pipeline it feeds). Returns false (error
 // recorded) if a wait ran out.
 template <typename T, bool RESID>
-__device__ __noinline__ bool sweep_tma(block_view<T> in, block_view<T> out, int w, int h, void* smem,
+__device__ bool sweep_tma(block_view<T> in, block_view<T> out, int w, int h, void* smem,
     size_t smem_bytes, const tma_plan& P, double* acc_out) {
   constexpr int V = traits<T>::VEC;
   constexpr int H = V;  // halo elements each side of a slot row (16 bytes)
@@ -870,15 +870,17 @@ __device__ __noinline__ bool sweep_tma(block_view<T> in, block_view<T> out, int 
   }
   __syncthreads();
 
-  long long issued = 0;  // producer state (lane 0 of warp 0)
+  // producer state (lane 0 of warp 0): rows issued, and the next one's slot,
+  // round of the ring, tile and row, found by counting (the divisions by the
+  // slot count and the rows were most of a row's instructions)
+  long long issued = 0;
+  int is = 0, iu = 0, it = 0, ir = 0;
   auto try_issue = [&]() {
     while (issued < total) {
-      long long j = issued;
-      int s = (int)(j % P.NS);
-      long long u = j / P.NS;
-      if (u > 0 && !mbar_test_wait(&empty[s], (unsigned)((u - 1) & 1))) break;
-      int t = (int)(j / rows), r = (int)(j % rows);
-      int c0 = t * P.tws;
+      const long long j = issued;
+      const int s = is, r = ir;
+      if (iu > 0 && !mbar_test_wait(&empty[s], (unsigned)((iu - 1) & 1))) break;
+      int c0 = it * P.tws;
       int tw = min(P.tws, w - c0);
       unsigned bytes = (unsigned)(((size_t)(tw + 2 * H) * sizeof(T) + 15) / 16 * 16);
       // checked build: 16-byte aligned source, copy fits its slot
@@ -890,6 +892,14 @@ __device__ __noinline__ bool sweep_tma(block_view<T> in, block_view<T> out, int 
       bulk_g2s(slots + (size_t)s * P.slot_elems, in.row(r) + traits<T>::OFF + c0 - H, bytes,
                &full[s]);
       issued = j + 1;
+      if (++is == P.NS) {
+        is = 0;
+        iu++;
+      }
+      if (++ir == rows) {
+        ir = 0;
+        it++;
+      }
     }
   };
   const bool producer = (warp == 0 && lane == 0);
@@ -901,19 +911,18 @@ __device__ __noinline__ bool sweep_tma(block_view<T> in, block_view<T> out, int 
 
   double acc = 0.0;
   bool fail = false;
+  int sc = 0, s1 = 0, s2 = 0;  // slots of the current row and of the two before it
+  unsigned parity = 0;
   for (int t = 0; t < P.ntiles && !fail; t++) {
     const int c0 = t * P.tws;
     const int tw = min(P.tws, w - c0);
-    const long long ibase = (long long)t * rows;
     const int v = warp * 32 + lane;      // vector of the tile row this lane owns
     const bool active = v * V < tw;
     const bool next_active = (v + 1) * V < tw;
     const int nvalid = active ? min(V, tw - v * V) : 0;
     const int s_off = H + v * V;         // slot element of interior column c0 + v*V
     for (int r = 0; r < rows; r++) {
-      const long long j = ibase + r;
-      const unsigned parity = (unsigned)((j / P.NS) & 1);
-      unsigned long long* fb = &full[j % P.NS];
+      unsigned long long* fb = &full[sc];
       unsigned spins = 0;
       while (true) {
         // The producer's warp must not be suspended inside try_wait while
@@ -929,9 +938,9 @@ __device__ __noinline__ bool sweep_tma(block_view<T> in, block_view<T> out, int 
       }
       if (fail) break;
       if (r >= 2) {
-        const T* up = slots + (size_t)((j - 2) % P.NS) * P.slot_elems;
-        const T* mid = slots + (size_t)((j - 1) % P.NS) * P.slot_elems;
-        const T* dn = slots + (size_t)(j % P.NS) * P.slot_elems;
+        const T* up = slots + s2 * P.slot_elems;
+        const T* mid = slots + s1 * P.slot_elems;
+        const T* dn = slots + sc * P.slot_elems;
         T m[V];
         if (active) {
           if (V == 2) {
@@ -955,15 +964,21 @@ __device__ __noinline__ bool sweep_tma(block_view<T> in, block_view<T> out, int 
                                        out.at(r - 1, 1 + c0 + v * V), nvalid);
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[(j - 2) % P.NS]);
+        if (lane == 0) mbar_arrive(&empty[s2]);
         if (producer) try_issue();
+      }
+      s2 = s1;
+      s1 = sc;
+      if (++sc == P.NS) {
+        sc = 0;
+        parity ^= 1;
       }
     }
     if (!fail) {
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(&empty[(ibase + h) % P.NS]);
-        mbar_arrive(&empty[(ibase + h + 1) % P.NS]);
+        mbar_arrive(&empty[s2]);  // rows h and h + 1
+        mbar_arrive(&empty[s1]);
       }
     }
   }
