@@ -391,7 +391,8 @@ __device__ __noinline__ void put_rects(int n, int src_pitch, int t, int nt) {
 // taken by warp 0 while the other warps copy. All threads. On the headline
 // decomposition (2048 x 221 chares, 6 sweeps per pass) the halos of a pass
 // took about 105 us of 384 when they were packed into the ring, unpacked and
-// delivered to the block one by one, and take about 60 this way.
+// delivered to the block one by one; all of a pass beside its sweeps takes
+// about 50 us of 302 this way, the puts themselves 17.
 template <typename T>
 __device__ void put_halos(JBlock& c, const jac::chare_desc& d, int phase) {
   constexpr int V = jac::traits<T>::VEC;

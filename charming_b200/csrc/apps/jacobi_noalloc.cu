@@ -75,8 +75,8 @@ int scratch_on_current_device(void** out, int* sms) {
 // NA_U rows are in flight in registers. FIX: the item's levels can meet the
 // boundary ring. The grids stay in L2; small ones are bound by the launch and
 // the chain of a warp's rows, large ones by instruction issue. 254^2 FP64, 20
-// sweeps: 96 us with one launch per sweep (two copies, a 64-bit division per
-// point); 2046^2 FP32, 100 sweeps: 1870 us.
+// sweeps: 34 us (96 with one launch per sweep, two copies and a 64-bit division
+// per point); 2046^2 FP32, 100 sweeps: 320 us (1870 so).
 constexpr int NA_U = 4;
 
 template <typename T, int L, bool ALIGNED, bool FIX>
