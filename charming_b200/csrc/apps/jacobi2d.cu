@@ -342,6 +342,8 @@ __shared__ put_batch s_puts;
 
 // Rectangle k of the batch, by threads t of nt: the loads of four units are in
 // flight together; a thread's next unit is found by adding, not dividing.
+// A side halo runs over all rows of a chare, whose grid may hold more than
+// 2^31 elements: row offsets are 64-bit.
 template <typename T, typename U>
 __device__ __forceinline__ void put_one(const put_batch& b, int k, int src_pitch, int t, int nt) {
   constexpr int B = 4, W = sizeof(U) / sizeof(T);
@@ -352,11 +354,11 @@ __device__ __forceinline__ void put_one(const put_batch& b, int k, int src_pitch
   const int dr = nt / nu, dx = nt - dr * nu;
   for (int i = t; i < total; i += B * nt) {
     U v[B];
-    int off[B];
+    long long off[B];
 #pragma unroll
     for (int q = 0; q < B; q++) {
-      if (i + q * nt < total) v[q] = *reinterpret_cast<const U*>(src + r * src_pitch + x * W);
-      off[q] = r * dst_pitch + x * W;
+      if (i + q * nt < total) v[q] = *reinterpret_cast<const U*>(src + (long long)r * src_pitch + x * W);
+      off[q] = (long long)r * dst_pitch + x * W;
       r += dr;
       x += dx;
       if (x >= nu) {

@@ -131,3 +131,10 @@ def test_chare_code_threaded_block(emu, cfg):
     assert int(f["done"]) == px * py
     if K > 0:
         assert int(f["sweeps"]) == expected_stop(nx, ny, K, tol, ms, bc, dt)
+
+
+def test_halo_puts_address_large_grids(emu):
+    """Side halos of a grid of more than 2^31 elements: every cell arrives at
+    its 64-bit offset, by vectors and by elements (tests/emu/put_test.cpp)."""
+    r = subprocess.run([os.path.join(os.path.dirname(emu), "put_test")], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stdout[-1000:], r.stderr[-1000:])
