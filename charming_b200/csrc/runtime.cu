@@ -961,6 +961,18 @@ __device__ __forceinline__ chare_proxy_base* proxy_of(pe_state* ps, int cid) {
   return (cid >= 0 && cid < tb.count) ? tb.proxies[cid] : nullptr;
 }
 
+// One thread: whether the stash has a descriptor and arena space for a message
+// of `bytes`; *at: where in the arena.
+__device__ bool stash_fits(unsigned long long bytes, unsigned long long* at) {
+  pe_state* ps = pes();
+  const unsigned long long A = c_rt.stash_bytes;
+  unsigned long long v = ps->arena_tail;
+  const unsigned long long p = v % A;
+  if (p + bytes > A) v += A - p;
+  *at = v;
+  return ps->key_tail - ps->key_head < (unsigned long long)c_rt.stash_entries && v + bytes - ps->arena_head <= A;
+}
+
 // Thread 0: a stash descriptor and arena space for a message of `bytes`;
 // the arena address, or nullptr (error recorded).
 __device__ unsigned char* stash_alloc(unsigned long long bytes, int chare_id, int chare_idx, int refnum,
@@ -968,12 +980,8 @@ __device__ unsigned char* stash_alloc(unsigned long long bytes, int chare_id, in
   pe_state* ps = pes();
   const unsigned long long S = (unsigned long long)c_rt.stash_entries;
   const unsigned long long A = c_rt.stash_bytes;
-  bool ok = ps->key_tail - ps->key_head < S;
-  unsigned long long v = ps->arena_tail;
-  const unsigned long long p = v % A;
-  if (p + bytes > A) v += A - p;
-  if (v + bytes - ps->arena_head > A) ok = false;
-  if (!ok) {
+  unsigned long long v = 0;
+  if (!stash_fits(bytes, &v)) {
     set_error(CHARMING_ERR_STASH_FULL, (int)(ps->key_tail - ps->key_head), (int)bytes);
     return nullptr;
   }
@@ -1594,17 +1602,19 @@ __device__ void batch_extend() {
     const int bi = __shfl_sync(FULL, w0 ? lo.idx : hi.idx, src);
     const int be = __shfl_sync(FULL, w0 ? lo.ep : hi.ep, src);
     if (kind == 2) {  // its stash descriptor and arena space, by lane 0
-      unsigned long long dst = 0;
+      // (with no room it ends the batch: what the batch delivers may make some)
+      unsigned long long dst = 0, at = 0;
       unsigned char* m = reinterpret_cast<unsigned char*>(ba) - HDR;
       if (lane == 0) {
         const envelope* env = reinterpret_cast<const envelope*>(m);
         const regular_msg* rm = reinterpret_cast<const regular_msg*>(m + sizeof(envelope));
-        dst = reinterpret_cast<unsigned long long>(stash_alloc(env->size, rm->chare_id, bi, rm->refnum, env->src_pe));
+        if (stash_fits(env->size, &at))
+          dst = reinterpret_cast<unsigned long long>(stash_alloc(env->size, rm->chare_id, bi, rm->refnum, env->src_pe));
         ps->bdst[n] = reinterpret_cast<void*>(dst);
         ps->barg[n] = m;
         ps->bbytes[n] = (unsigned int)env->size;
       }
-      if (!__shfl_sync(FULL, dst, 0)) break;  // stash full: error recorded
+      if (!__shfl_sync(FULL, dst, 0)) break;
       early |= 1u << n;
     } else if (lane == n) {
       mkey = k;

@@ -13,6 +13,7 @@
 // RT_EMU_RANK=r and RT_EMU_DIR=<empty directory> run w processes, one GPU
 // each, whose inbox sides are files every process maps shared (in the role
 // of CUDA IPC), bootstrapped by the process main's file rendezvous.
+// RT_EMU_STASH_ENTRIES=n: a stash of n messages per PE.
 // usage (n_pes: PE blocks; with RT_EMU_GPU_LEVEL set they form one PE):
 //        rt_emu fanout n_pes ring_bytes n_chares msgs payload seed mode
 //        rt_emu hello n_pes ring_bytes
@@ -274,7 +275,7 @@ void init_runtime(int n_blocks, size_t ring_bytes, bool gpu_level) {
   ds.max_msg = 4096 + 64;
   ds.ring_stride = ds.ring_cells * CELL + ds.max_msg;
   ds.stash_bytes = 4 << 20;
-  ds.stash_entries = 4096;
+  ds.stash_entries = env_int("RT_EMU_STASH_ENTRIES", 4096);
   ds.smem_state_bytes = (int)((sizeof(pe_state) + 8ull * n_pes + 127) / 128 * 128);
   ds.smem_total = SMEM_BYTES;
   ds.smem_arena_bytes = 8 << 10;

@@ -28,9 +28,9 @@ def emus():
     return {k: os.path.join(OUT, k) for k in ("rt_emu", "rt_emu_tsan", "rt_emu_mt")}
 
 
-def run(exe, args, threads=1, timeout=600):
+def run(exe, args, threads=1, timeout=600, **extra_env):
     env = dict(os.environ, ASAN_OPTIONS="detect_leaks=0", TSAN_OPTIONS="halt_on_error=1",
-               RT_EMU_THREADS=str(threads))
+               RT_EMU_THREADS=str(threads), **extra_env)
     r = subprocess.run([exe] + [str(a) for a in args], capture_output=True, text=True,
                        timeout=timeout, env=env)
     assert "ThreadSanitizer" not in r.stderr and "divergence" not in r.stderr, r.stderr[-3000:]
@@ -97,6 +97,59 @@ def test_warp_entry_methods_run_in_batches(emus, threads, n, msgs, payload, mode
     chk = msgmodel.check_fanout_log(log, n, msgs, payload, 0xBA7 + n + mode, mode)
     assert chk.ok, chk.errors
     assert int(head.split("batched=")[1].split()[0]) > 0
+
+
+def stash_need(n, msgs, seed):
+    """Stash entries that the fan-out with refnums needs on one PE that takes
+    its messages one at a time, ready stashed ones first (the span from the
+    oldest entry still held to the newest). All messages reach the PE in
+    sending order."""
+    dst = msgmodel.fanout_destinations(n, msgs, seed).reshape(-1)
+    order = [(int(d), j % msgs) for j, d in enumerate(dst)]
+    left = [[0] * (msgs + 1) for _ in range(n)]
+    for d, k in order:
+        left[d][k] += 1
+    cur = [0] * n
+
+    def settle(d):
+        while cur[d] < msgs and left[d][cur[d]] == 0:
+            cur[d] += 1
+    for d in range(n):
+        settle(d)
+    stash, head, need = [], 0, 0  # None: freed
+    for d, k in order:
+        if k != cur[d]:
+            stash.append((d, k))
+            need = max(need, len(stash) - head)
+            continue
+        left[d][k] -= 1
+        settle(d)
+        while True:  # the oldest ready one, until none is
+            i = next((j for j in range(head, len(stash)) if stash[j] and stash[j][1] == cur[stash[j][0]]), None)
+            if i is None:
+                break
+            e, r = stash[i]
+            stash[i] = None
+            left[e][r] -= 1
+            settle(e)
+            while head < len(stash) and stash[head] is None:
+                head += 1
+    assert head == len(stash) and not any(map(any, left))
+    return need
+
+
+@pytest.mark.parametrize("threads", [64, 128])
+@pytest.mark.parametrize("n,msgs,seed", [  # seeds with an early message behind the delivery that makes room
+    (3, 4, 100), (6, 6, 35), (8, 8, 9), (12, 6, 42), (16, 8, 51), (40, 16, 1)])
+def test_batches_need_no_larger_stash(emus, threads, n, msgs, seed):
+    """Early messages that a batch takes along go to the stash before the
+    batch's deliveries make room there: with a stash that just holds what the
+    messages need one at a time, they must wait in the ring instead of
+    failing the run."""
+    r = run(emus["rt_emu_mt"], ["fanout", 1, 1 << 20, n, msgs, 64, seed, 1], threads,
+            RT_EMU_STASH_ENTRIES=str(stash_need(n, msgs, seed)))
+    head = r.stdout.splitlines()[0]
+    assert r.returncode == 0 and head.startswith("status=0"), (head, r.stderr[-2000:])
 
 
 @pytest.mark.parametrize("exe,n_pes,threads,ring,n,msgs,payload,mode", [
