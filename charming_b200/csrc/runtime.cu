@@ -1346,7 +1346,8 @@ __device__ void stash_batch(chare_proxy_base* p, int cid, int idx, int ep, void*
 
 // Thread 0: runs entry method *ep of chare idx here if it is an inline one.
 // True when the delivery ended with it; else *ep is the entry method that the
-// block has to run.
+// block has to run. A returned number that is no block or warp-level entry
+// method of the proxy is an error (it would be called through the table).
 __device__ bool inline_done(pe_state* ps, chare_proxy_base* p, int idx, int* ep, void* arg) {
   if (!p->inline_em(*ep)) return false;
   const long long c0 = clock64();
@@ -1354,6 +1355,10 @@ __device__ bool inline_done(pe_state* ps, chare_proxy_base* p, int idx, int* ep,
   ps->stats[ST_EM_CYC] += (unsigned long long)(clock64() - c0);
   if (next < 0) {
     if ((++ps->stats[ST_DELIVERED] & 15) == 0) stamp_progress(ps->my_pe);
+    return true;
+  }
+  if (!p->valid_target(idx, next) || p->inline_em(next)) {
+    set_error(CHARMING_ERR_BAD_TARGET, p->id, next);
     return true;
   }
   *ep = next;

@@ -134,7 +134,8 @@ struct chare_proxy_base {
   // block). The scheduler decides the refnum match (refnum_matches, the
   // rule of include/chare.h:181-195) in one thread before it calls: the
   // entry method may change the chare's refnum at once, so the threads must
-  // not test it again here. Returns true.
+  // not test it again here. Returns true (false, with BAD_TARGET, for an
+  // inline entry method).
   __device__ virtual bool call(int idx, int ep, void* arg, int ref) = 0;
   // Frees the local chares and tables (the runtime calls it when a run ends
   // and then deletes the proxy).
@@ -260,10 +261,10 @@ struct chare_proxy : chare_proxy_base {
   // itself, without the block (an extension, for small bookkeeping
   // deliveries: a block delivery costs its barriers and the register frames
   // of every thread). It must not synchronise and sends with invoke_single
-  // only. It returns the number of a block entry method of the same chare
-  // array that the block is to run next on this chare with the same
-  // argument, or -1 when the delivery is done. Single-threaded, like
-  // add_entry_method.
+  // only. It returns the number of a block or warp-level entry method of the
+  // same chare array that is to run next on this chare with the same
+  // argument, or -1 when the delivery is done; any other number ends the run
+  // with BAD_TARGET. Single-threaded, like add_entry_method.
   template <int Func(C&, void*)>
   __device__ static int em_inline_entry(chare_proxy_base* base, int idx, void* arg) {
     chare_proxy<C>* self = static_cast<chare_proxy<C>*>(base);
@@ -281,6 +282,10 @@ struct chare_proxy : chare_proxy_base {
 
   __device__ static bool call_static(chare_proxy_base* base, int idx, int ep, void* arg) {
     chare_proxy<C>* self = static_cast<chare_proxy<C>*>(base);
+    if (self->inline_em(ep)) {  // the scheduler's thread 0 alone runs those
+      if (threadIdx.x == 0) detail::report_error(detail::ERR_BAD_TARGET, self->id, ep);
+      return false;
+    }
     self->em_tab[ep](base, idx, arg);
     return true;
   }

@@ -18,6 +18,7 @@
 //        rt_emu fanout n_pes ring_bytes n_chares msgs payload seed mode
 //        rt_emu hello n_pes ring_bytes
 //        rt_emu refnum n_pes ring_bytes reversed
+//        rt_emu inline n_pes ring_bytes n_chares msgs refnums kind
 //        rt_emu serve n_pes ring_bytes n_requests seed workers_per_pe
 //               max_inflight chare_side dtype(0 f64, 1 f32)
 // serve runs the Jacobi2d solve server (apps/jacobi2d.cu in serving mode,
@@ -193,8 +194,143 @@ int fanout_plan(int n, int msgs, unsigned long long seed, std::vector<int>& expe
 extern "C" int oracle_jacobi2d_f32(float* grid, int nx, int ny, int sweeps, int threads);
 
 // programs of the library that this check does not run
-__device__ void suite::jacobi1d_main(int) { charm::end(); }
 __device__ void suite::serve_main(int) { charm::end(); }
+
+// ---- inline entry methods (in the place of the library's jacobi1d) ----------
+// n chares send m messages each; message k of chare s goes to chare
+// (s + k) % n with refnum R - 1 - k / (m / R), so all but the last m / R of a
+// sender are early. The receiving entry method counts up its chare's refnum
+// after the m / R messages that it gets of each. kind 0: it is an inline one,
+// which hands every third delivery to a block and every third to a warp-level
+// entry method; kind 1: a warp-level one; 2: an inline one that returns a
+// number past the last entry method, 3: one that returns an inline one's.
+// With kind 0 a chare that has everything waits (async_wait, an inline entry
+// method) until its predecessor has, and the woken ones report to chare 0.
+// g_app: a[0] n, a[1] m, a[2] R, a[3] kind; p[0] log (u32[n][m][4]: sender, k,
+// refnum, route), p[1] counters (u64: chares done, block and warp runs, notes
+// of the block runs), p[2] signal words (u64[n])
+namespace {
+enum : int { EP_L_START, EP_L_TAKE, EP_L_BLOCK, EP_L_WARP, EP_L_WOKEN, EP_L_DONE, EP_L_END, EP_L_NOTE };
+struct LChare : charm::chare {
+  int ref, got, seq, done, notes;
+  __device__ LChare() : ref(0), got(0), seq(0), done(0), notes(0) {}
+};
+__shared__ charm::chare_proxy<LChare>* l_proxy;
+unsigned int* l_log(const LChare& c, int at) {
+  return static_cast<unsigned int*>(g_app.p[0]) + 4 * ((size_t)c.i * (size_t)g_app.a[1] + (size_t)at);
+}
+unsigned long long* l_ctr(int k) { return static_cast<unsigned long long*>(g_app.p[1]) + k; }
+
+void l_start(LChare& c, void*) {
+  const int n = (int)g_app.a[0], m = (int)g_app.a[1], R = (int)g_app.a[2];
+  __shared__ int pay[4];
+  for (int k = 0; k < m; k++) {
+    const int ref = R - 1 - k / (m / R);
+    if (threadIdx.x == 0) {
+      pay[0] = c.i;
+      pay[1] = k;
+      pay[2] = ref;
+    }
+    __syncthreads();
+    int b[4] = {pay[0], pay[1], pay[2], 0};
+    l_proxy->invoke((c.i + k) % n, EP_L_TAKE, b, sizeof(b), ref);
+  }
+}
+// One thread: the record of a delivery; its place in the chare's order.
+int l_record(LChare& c, const void* arg, int route) {
+  const int* b = static_cast<const int*>(arg);
+  const int at = c.seq++;
+  unsigned int* r = l_log(c, at);
+  r[0] = (unsigned)b[0];
+  r[1] = (unsigned)b[1];
+  r[2] = (unsigned)b[2];
+  r[3] = (unsigned)route;
+  const int m = (int)g_app.a[1], R = (int)g_app.a[2];
+  if (++c.got == m / R) {
+    c.got = 0;
+    l_proxy->set_refnum(c.i, ++c.ref);
+  }
+  return at;
+}
+int l_take(LChare& c, void* arg) {
+  const int kind = (int)g_app.a[3], m = (int)g_app.a[1];
+  const int at = l_record(c, arg, 0);
+  if (kind == 2) return EP_L_NOTE + 1;
+  if (kind == 3) return EP_L_TAKE;
+  if (c.seq == m) {
+    uint64_t* sig = static_cast<uint64_t*>(g_app.p[2]);
+    l_proxy->async_wait(sig + c.i, 1, charm::CMP_GE, 1, c.i, EP_L_WOKEN);
+    if (c.i == 0) charm::rt::st_release_u64(reinterpret_cast<unsigned long long*>(sig), 1);
+  }
+  return at % 3 == 1 ? EP_L_BLOCK : at % 3 == 2 ? EP_L_WARP : -1;
+}
+void l_block(LChare& c, void* arg) {
+  if (threadIdx.x == 0) {
+    const int* b = static_cast<const int*>(arg);
+    unsigned int* r = l_log(c, c.seq - 1);
+    if (r[0] == (unsigned)b[0] && r[1] == (unsigned)b[1]) r[3] |= 1;
+    atomicAdd(l_ctr(1), 1ULL);
+    l_proxy->invoke_single(0, EP_L_NOTE, nullptr, 0);
+  }
+}
+void l_warp(LChare& c, void* arg) {
+  if ((threadIdx.x & 31) == 0) {
+    if (g_app.a[3] == 1) {
+      l_record(c, arg, 4);
+      if (c.seq == (int)g_app.a[1] && atomicAdd(l_ctr(0), 1ULL) + 1 == (unsigned long long)g_app.a[0]) charm::end();
+      return;
+    }
+    const int* b = static_cast<const int*>(arg);
+    unsigned int* r = l_log(c, c.seq - 1);
+    if (r[0] == (unsigned)b[0] && r[1] == (unsigned)b[1]) r[3] |= 2;
+    atomicAdd(l_ctr(2), 1ULL);
+  }
+}
+int l_woken(LChare& c, void* arg) {
+  uint64_t* sig = static_cast<uint64_t*>(g_app.p[2]);
+  if (arg == nullptr && c.i + 1 < (int)g_app.a[0])
+    charm::rt::st_release_u64(reinterpret_cast<unsigned long long*>(sig + c.i + 1), 1);
+  l_proxy->invoke_single(0, EP_L_DONE, nullptr, 0);
+  return -1;
+}
+// Chare 0: ends the run when every chare is done and the block runs' notes are in.
+int l_finish(LChare& c) {
+  const int n = (int)g_app.a[0], m = (int)g_app.a[1];
+  if (c.done < n || c.notes < n * ((m + 1) / 3)) return -1;
+  *l_ctr(0) = (unsigned long long)c.done;
+  *l_ctr(3) = (unsigned long long)c.notes;
+  return EP_L_END;
+}
+int l_done(LChare& c, void*) {
+  c.done++;
+  return l_finish(c);
+}
+int l_note(LChare& c, void*) {
+  c.notes++;
+  return l_finish(c);
+}
+void l_end(LChare&, void*) { charm::end(); }
+}  // namespace
+
+__device__ void suite::jacobi1d_main(int) {
+  if (threadIdx.x == 0) {
+    l_proxy = new charm::chare_proxy<LChare>();
+    l_proxy->add_entry_method<&l_start>();
+    if (g_app.a[3] == 1) l_proxy->add_warp_entry_method<&l_warp>();
+    else l_proxy->add_inline_entry_method<&l_take>();
+    l_proxy->add_entry_method<&l_block>();
+    l_proxy->add_warp_entry_method<&l_warp>();
+    l_proxy->add_inline_entry_method<&l_woken>();
+    l_proxy->add_inline_entry_method<&l_done>();
+    l_proxy->add_entry_method<&l_end>();
+    l_proxy->add_inline_entry_method<&l_note>();
+    l_proxy->create((int)g_app.a[0]);
+    for (int c = l_proxy->start_idx; l_proxy->n_local > 0 && c <= l_proxy->end_idx; c++) l_proxy->set_refnum(c, 0);
+  }
+  __syncthreads();
+  for (int c = l_proxy->start_idx; l_proxy->n_local > 0 && c <= l_proxy->end_idx; c++)
+    l_proxy->invoke(c, EP_L_START);
+}
 
 namespace {
 
@@ -666,6 +802,23 @@ int main(int argc, char** argv) {
     printf("status=%d order=", status);
     for (int v : order) printf("%d,", v);
     printf("\n");
+    return 0;
+  }
+  if (app == "inline") {
+    if (argc < 8) return 2;
+    const int n = atoi(argv[4]), m = atoi(argv[5]);
+    std::vector<unsigned int> log(4 * (size_t)n * m, ~0u);
+    std::vector<unsigned long long> ctr(8, 0), sig(n, 0);
+    g_app.id = suite::APP_JACOBI1D;
+    for (int k = 0; k < 4; k++) g_app.a[k] = atoi(argv[4 + k]);
+    g_app.p[0] = log.data();
+    g_app.p[1] = ctr.data();
+    g_app.p[2] = sig.data();
+    const int status = run_scheduler(n_pes, threads);
+    printf("status=%d done=%llu block=%llu warp=%llu notes=%llu batched=%llu\n", status, ctr[0], ctr[1], ctr[2],
+           ctr[3], g_batched);
+    for (size_t r = 0; r < (size_t)n * m; r++)
+      printf("L %u %u %u %u\n", log[4 * r], log[4 * r + 1], log[4 * r + 2], log[4 * r + 3]);
     return 0;
   }
   if (app == "decomp1d") {  // rt_emu decomp1d n_pes ring_bytes n_chares nx ny iters mode

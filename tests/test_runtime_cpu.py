@@ -168,6 +168,53 @@ def test_full_rings_defer_sends_instead_of_deadlock(emus, exe, n_pes, threads, r
     assert deferred > 0
 
 
+def ladder(exe, n_pes, threads, n, m, refs, kind, ring=1 << 20):
+    """The inline / warp-level refnum ladder of rt_emu: its counters, after
+    checking each chare's log: refnums in order, of one refnum each sender's
+    messages in order, each message once."""
+    r = run(exe, ["inline", n_pes, ring, n, m, refs, kind], threads)
+    head = dict(kv.split("=") for kv in r.stdout.splitlines()[0].split())
+    if head["status"] != "0":
+        return head
+    log = np.array([l.split()[1:] for l in r.stdout.splitlines() if l.startswith("L ")], dtype=np.int64).reshape(n, m, 4)
+    for d in range(n):
+        src, k, ref, route = log[d].T
+        assert np.array_equal(ref, np.repeat(np.arange(refs), m // refs))
+        assert np.array_equal(ref, refs - 1 - k // (m // refs)) and np.array_equal((src + k) % n, np.full(m, d))
+        assert len(set(zip(src, k))) == m
+        for a in range(n):
+            for q in range(refs):
+                assert np.all(np.diff(k[(src == a) & (ref == q)]) > 0)
+        assert np.array_equal(route, np.arange(m) % 3 if kind == 0 else np.full(m, 4))
+    return {k: int(v) for k, v in head.items()}
+
+
+@pytest.mark.parametrize("exe,n_pes,threads,n,m,refs", [
+    ("rt_emu", 4, 1, 12, 24, 4),       # early messages of inline entry methods through the stash
+    ("rt_emu_tsan", 3, 1, 9, 27, 3),
+    ("rt_emu_mt", 1, 64, 6, 24, 4),    # and handed to the block and to warps
+    ("rt_emu_mt", 1, 32, 8, 8, 8),     # no batches on one warp
+    ("rt_emu", 1, 1, 4, 800, 5),       # 160 ready messages a chare: more than the ready list's records
+    ("rt_emu_mt", 1, 64, 3, 900, 3),   # 300: more than the ready list
+])
+def test_inline_entry_methods(emus, exe, n_pes, threads, n, m, refs):
+    """Inline entry methods from the inbox, from the stash (they move their
+    chare's refnum on) and from async_wait; what they return runs next on the
+    same chare and message, block-wide or on one warp."""
+    h = ladder(emus[exe], n_pes, threads, n, m, refs, 0)
+    assert h["status"] == 0 and h["done"] == n
+    assert h["block"] == h["notes"] == n * ((m + 1) // 3)
+    assert h["warp"] == n * (m // 3)
+
+
+@pytest.mark.parametrize("kind", [2, 3])
+@pytest.mark.parametrize("exe,threads", [("rt_emu", 1), ("rt_emu_mt", 64)])
+def test_inline_entry_method_returning_no_block_entry_method(emus, exe, threads, kind):
+    """A number past the last entry method, or that of an inline one: the run
+    ends with BAD_TARGET instead of a call through a wrong pointer."""
+    assert ladder(emus[exe], 1, threads, 4, 4, 2, kind)["status"] == "3"
+
+
 @pytest.mark.parametrize("reversed_order", [0, 1])
 @pytest.mark.parametrize("exe,n_pes,threads", [("rt_emu", 6, 1), ("rt_emu_mt", 1, 64)])
 def test_refnum_scenario(emus, exe, n_pes, threads, reversed_order):
