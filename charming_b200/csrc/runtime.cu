@@ -663,6 +663,8 @@ __device__ void charm::send_reg_msg(int chare_id, int chare_idx, int ep_id, void
 
 __device__ void charm::send_reg_msg_single(int chare_id, int chare_idx, int ep_id, const void* buf,
     size_t payload_size, int dst_pe, int refnum) {
+  // GPU-level mode: every block runs a block entry method, block 0 sends
+  if (gpu_level() && blockIdx.x != 0) return;
   pe_state* ps = pes();
   const unsigned long long bytes = envelope::alloc_size(msgtype::regular, payload_size);
   unsigned long long t = 0;

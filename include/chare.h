@@ -383,7 +383,8 @@ struct chare_proxy : chare_proxy_base {
   }
 
   // Single-threaded: from inline entry methods, or one thread (thread 0) of
-  // a block entry method.
+  // a block entry method (in GPU-level mode, where every block runs those,
+  // of block 0: the others' calls send nothing).
   inline __device__ void invoke_single(int idx, int ep, const void* buf, size_t size, int ref = -1) {
     if (idx < 0 || idx >= n_total) {
       detail::report_error(detail::ERR_BAD_TARGET, id, idx);

@@ -116,3 +116,25 @@ def test_gpu_level_program_runs(tmp_path):
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
     assert "GPU-level mode: 1 PE of" in r.stdout
     assert "gpu-level forms: pe 0 of 1, rounds 6, hits 3, bad 0" in r.stdout, r.stdout[-2000:]
+
+
+@pytest.mark.parametrize("mode", ["", "-DCHARMING_GPU_LEVEL"])
+def test_inline_entry_methods_program(tmp_path, mode):
+    """Inline entry methods reached from the inbox, the stash and async_wait,
+    handing messages on to the block, and invoke_single, in both modes
+    (tests/compile/inline_forms.cu)."""
+    arch = "-gencode arch=compute_100a,code=sm_100a"
+    lib = os.path.join(ROOT, "charming_b200", "lib", "libcharming.a")
+    src = os.path.join(ROOT, "tests", "compile", "inline_forms.cu")
+    obj, exe = tmp_path / "inl.o", tmp_path / "inl"
+    inc = os.path.join(ROOT, "include")
+    r = subprocess.run(f"nvcc -std=c++17 {arch} -rdc=true {mode} -I{inc} -c {src} -o {obj} && "
+                       f"nvcc {arch} -rdc=true -Xnvlink -suppress-stack-size-warning -o {exe} {obj} {lib} -lcudart",
+                       shell=True, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    env = dict(os.environ, CHARMING_DEADLINE_S="60", CHARMING_IDLE_TIMEOUT_S="3")
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120, env=env)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+    line = next(l for l in r.stdout.splitlines() if l.startswith("inline forms:"))
+    n = int(line.split("chares ")[1].split(",")[0])
+    assert line == f"inline forms: chares {n}, done {n}, notes {12 * n} of {12 * n}, bad 0"
