@@ -289,6 +289,7 @@ struct pe_state {
   void* bm_ptr[MSG_BATCH_MAX];
   unsigned long long bm_tick[MSG_BATCH_MAX];
   unsigned long long bm_bytes[MSG_BATCH_MAX];
+  int bm_ok;                           // all of them have space
   // followed by head_cache[n_pes] (unsigned long long), then scratch
 };
 

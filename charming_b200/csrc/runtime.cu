@@ -737,11 +737,25 @@ __device__ void charm::send_user_msg(int chare_id, int chare_idx, int ep_id,
   msg.env = nullptr;
 }
 
+namespace {
+__device__ __forceinline__ void fill_message(charm::message& m, unsigned char* at, unsigned long long ticket, int dst,
+    unsigned long long bytes) {
+  m.env = reinterpret_cast<envelope*>(at);
+  m.offset = ticket;
+  m.dst_pe = dst;
+  m.cells = (int)cells_for(bytes);
+  m.capacity = at ? (size_t)(bytes - HDR) : 0;
+}
+}  // namespace
+
 __device__ bool charm::alloc_user_msgs(message* msgs, const int* dst_pes,
     const size_t* payload_sizes, int n) {
   if (n > MSG_BATCH_MAX) n = MSG_BATCH_MAX;
   if (gpu_level()) return group_alloc_user_msgs(msgs, dst_pes, payload_sizes, n);
   pe_state* ps = pes();
+  // 512 private copies of the descriptors cost each batch about 300 KB of
+  // local-memory stores; a block-shared array has one
+  const bool shared = __isShared(msgs);
   if (blockDim.x >= 32) {
     // Warp 0, one lane per message. Lanes whose messages go to the same PE
     // form a group (__match_any_sync): its lowest lane takes the tickets of
@@ -776,18 +790,25 @@ __device__ bool charm::alloc_user_msgs(message* msgs, const int* dst_pes,
       // the outbox, which flushes strictly in entry order, so a group's
       // later ticket must never enter it before an earlier one. Lanes of
       // different groups wait together.
+      unsigned char* got = nullptr;
+      unsigned long long tick = 0;
       const int rank = __popc(grp & ((1u << k) - 1));
       int rounds = __popc(grp);
       for (int o = 16; o > 0; o >>= 1) rounds = max(rounds, __shfl_xor_sync(FULL, rounds, o));
       for (int r = 0; r < rounds; r++) {
         if (act && rank == r) {
-          unsigned long long t = 0;
-          ps->bm_ptr[k] = ok ? wait_space(dst_pes[k], base + pre, bytes, &t) : nullptr;
-          ps->bm_tick[k] = t;
+          got = ok ? wait_space(dst_pes[k], base + pre, bytes, &tick) : nullptr;
+          ps->bm_ptr[k] = got;
+          ps->bm_tick[k] = tick;
           ps->bm_bytes[k] = bytes;
         }
         __syncwarp();
       }
+      // a block-shared array (block_messages()) is filled here, each
+      // descriptor by its lane
+      if (shared && act) fill_message(msgs[k], got, tick, dst_pes[k], bytes);
+      const bool all = __all_sync(FULL, !act || got != nullptr);
+      if (k == 0) ps->bm_ok = all ? 1 : 0;
       CHARM_PROF(__syncwarp(); if (k == 0) {
         ps->stats[ST_TICKET_NS] += tb - ta;
         ps->stats[ST_SPACE_NS] += globaltimer() - tb;
@@ -804,20 +825,17 @@ __device__ bool charm::alloc_user_msgs(message* msgs, const int* dst_pes,
     }
   }
   __syncthreads();
-  // every thread's own array, or a block-shared one (block_messages()) that
-  // thread 0 fills: 512 private copies of the descriptors cost each batch
-  // about 300 KB of local-memory stores
-  const bool fill = !__isShared(msgs) || threadIdx.x == 0;
   bool ok = true;
-  for (int j = 0; j < n; j++) {
-    if (fill) {
-      msgs[j].env = reinterpret_cast<envelope*>(ps->bm_ptr[j]);
-      msgs[j].offset = ps->bm_tick[j];
-      msgs[j].dst_pe = dst_pes[j];
-      msgs[j].cells = (int)cells_for(ps->bm_bytes[j]);
-      msgs[j].capacity = ps->bm_ptr[j] ? (size_t)(ps->bm_bytes[j] - HDR) : 0;
+  if (shared && blockDim.x >= 32) {
+    ok = ps->bm_ok != 0;
+  } else {
+    // every thread's own array (a block-shared one: thread 0 fills it)
+    const bool fill = !shared || threadIdx.x == 0;
+    for (int j = 0; j < n; j++) {
+      if (fill)
+        fill_message(msgs[j], static_cast<unsigned char*>(ps->bm_ptr[j]), ps->bm_tick[j], dst_pes[j], ps->bm_bytes[j]);
+      ok = ok && ps->bm_ptr[j] != nullptr;
     }
-    ok = ok && ps->bm_ptr[j] != nullptr;
   }
   __syncthreads();
   return ok;

@@ -99,6 +99,14 @@ def test_warp_entry_methods_run_in_batches(emus, threads, n, msgs, payload, mode
     assert int(head.split("batched=")[1].split()[0]) > 0
 
 
+@pytest.mark.parametrize("exe,threads", [("rt_emu", 1), ("rt_emu_mt", 32), ("rt_emu_mt", 96)])
+def test_batch_that_cannot_be_sent(emus, exe, threads):
+    """A batch of messages above the largest size: every thread of the block
+    learns that there is no space, and the run ends with MSG_TOO_LARGE."""
+    r = run(emus[exe], ["fanout", 1, 1 << 18, 6, 8, 8192, 3, 0], threads)
+    assert r.stdout.startswith("status=8 "), (r.stdout[:200], r.stderr[-2000:])
+
+
 def stash_need(n, msgs, seed):
     """Stash entries that the fan-out with refnums needs on one PE that takes
     its messages one at a time, ready stashed ones first (the span from the
