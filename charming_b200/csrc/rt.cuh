@@ -43,7 +43,9 @@ constexpr int HDR = 32;                  // envelope (16) + regular_msg (16)
 constexpr int MAX_THREADS = CHARMING_MAX_THREADS;  // launch bound of the scheduler
 constexpr int PROXY_CACHE = 16;          // proxies per PE looked up on chip
 constexpr int SMEM_OBJ_MAX = 4096;       // larger objects skip the on-chip arena
-constexpr int RQ_MAX = 128;              // ready stash entries listed on chip
+constexpr int RQ_MAX = 256;              // ready stash entries listed on chip,
+constexpr int RQ_REC = 128;              // ... so many of them with what their delivery needs
+constexpr unsigned int RQ_NO_REC = 255;  // the others' record number
 
 struct alignas(128) line_u64 {
   unsigned long long v;
@@ -234,11 +236,11 @@ struct pe_state {
   // ready stashed messages found by the last revive, in key order (offsets
   // from rq_base); rq_over: more than RQ_MAX, scan from ready_cursor instead
   unsigned long long rq_base;
-  // with what a delivery needs of each, read by the revive's threads together
-  // (rq: offset << 8 | record)
+  // (rq: offset << 8 | record, RQ_NO_REC: none, its key has the same); the
+  // records are read by the revive's threads together
   int rq_n, rq_pos, rq_over;
   unsigned int rq[RQ_MAX];
-  ready_rec rq_rec[RQ_MAX];
+  ready_rec rq_rec[RQ_REC];
   // block-collective broadcast slots
   void* b_ptr0;
   const void* b_ptr1;

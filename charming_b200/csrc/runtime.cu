@@ -1031,6 +1031,18 @@ __device__ void stash_retire() {
   if (ps->ready_cursor < ps->key_head) ps->ready_cursor = ps->key_head;
 }
 
+// What the delivery of a stashed message at arena offset off needs.
+__device__ __forceinline__ ready_rec record_of(const stash_key* k, unsigned long long off) {
+  const unsigned char* env = arena_of(blockIdx.x) + off;
+  ready_rec q;
+  q.idx = k->chare_idx;
+  q.refnum = k->refnum;
+  q.cid = (unsigned short)k->chare_id;  // (both below their table sizes)
+  q.ep = (unsigned short)reinterpret_cast<const regular_msg*>(env + sizeof(envelope))->ep_id;
+  q.off16 = (unsigned int)(off >> 4);
+  return q;
+}
+
 // Block-collective: waiting stashed messages whose refnum now matches become
 // ready (counted into red_i[0]), and every ready one goes on the on-chip
 // ready list (thread 0 sorts it before the next decision).
@@ -1053,15 +1065,10 @@ __device__ void stash_revive_scan() {
     if (st == KEY_READY) {
       const int pos = atomicAdd_block(&ps->rq_n, 1);
       const unsigned long long off = k->data_off % c_rt.stash_bytes;
-      if (pos < RQ_MAX && i - kh < (1ULL << 24) && off < (1ULL << 36)) {
-        const unsigned char* env = arena_of(blockIdx.x) + off;
-        ready_rec& q = ps->rq_rec[pos];
-        q.idx = k->chare_idx;
-        q.refnum = k->refnum;
-        q.cid = (unsigned short)k->chare_id;  // (both below their table sizes)
-        q.ep = (unsigned short)reinterpret_cast<const regular_msg*>(env + sizeof(envelope))->ep_id;
-        q.off16 = (unsigned int)(off >> 4);
-        ps->rq[pos] = (unsigned int)(i - kh) << 8 | (unsigned int)pos;
+      if (pos < RQ_MAX && i - kh < (1ULL << 24)) {
+        const bool rec = pos < RQ_REC && off < (1ULL << 36);
+        if (rec) ps->rq_rec[pos] = record_of(k, off);
+        ps->rq[pos] = (unsigned int)(i - kh) << 8 | (rec ? (unsigned int)pos : RQ_NO_REC);
       } else {
         atomicExch_block(&ps->rq_over, 1);
       }
@@ -1087,9 +1094,9 @@ __device__ void ready_list_sort() {
 }
 
 // Thread 0: the oldest ready stashed message, or ~0 when none is left:
-// from the ready list (*rec: its record there), or, when that overflowed, by
-// scanning the keys from ready_cursor (keys before it are known not to be
-// ready; *rec -1). A listed message stays ready until its delivery takes it
+// from the ready list (*rec: its record there, -1: it has none), or, when that
+// overflowed, by scanning the keys from ready_cursor (keys before it are known
+// not to be ready; *rec -1). A listed message stays ready until its delivery takes it
 // off the list, or until next_action puts it back to waiting.
 __device__ unsigned long long stash_next_ready(int* rec) {
   pe_state* ps = pes();
@@ -1098,7 +1105,7 @@ __device__ unsigned long long stash_next_ready(int* rec) {
   if (!ps->rq_over) {
     if (ps->rq_pos >= ps->rq_n) return ~0ULL;
     const unsigned int q = ps->rq[ps->rq_pos++];
-    *rec = (int)(q & 255);
+    *rec = (q & 255u) == RQ_NO_REC ? -1 : (int)(q & 255u);
     return ps->rq_base + (q >> 8);
   }
   *rec = -1;
@@ -1342,12 +1349,21 @@ __device__ void stash_batch(chare_proxy_base* p, int cid, int idx, int ep, void*
     const int pos = ps->rq_pos;
     int rec = 0;
     const unsigned long long j = stash_next_ready(&rec);  // (listed: rq_over takes no batch)
-    bool take = j != ~0ULL;
-    const ready_rec q = ps->rq_rec[rec];
-    chare_proxy_base* pj = take ? proxy_of(ps, q.cid) : nullptr;
+    if (j == ~0ULL) break;
+    ready_rec q;
+    unsigned long long off = 0;
+    if (rec >= 0) {
+      q = ps->rq_rec[rec];
+      off = (unsigned long long)q.off16 << 4;
+    } else {
+      const stash_key* k = keys_of(blockIdx.x) + j % (unsigned long long)c_rt.stash_entries;
+      off = k->data_off % c_rt.stash_bytes;
+      q = record_of(k, off);
+    }
+    chare_proxy_base* pj = proxy_of(ps, q.cid);
     const int idxj = q.idx, epj = q.ep;
     const unsigned long long key = ((unsigned long long)q.cid << 32) | (unsigned)idxj;
-    take = take && pj->warp_em(epj) && pj->refnum_matches(idxj, q.refnum);
+    bool take = pj->warp_em(epj) && pj->refnum_matches(idxj, q.refnum);
     for (int b = 0; take && b < ps->nb; b++) take = ps->bkeys[b] != key;
     if (!take) {  // leave it for the next decision
       ps->rq_pos = pos;
@@ -1357,7 +1373,7 @@ __device__ void stash_batch(chare_proxy_base* p, int cid, int idx, int ep, void*
     ps->bp[n] = pj;
     ps->bidx[n] = idxj;
     ps->bep[n] = epj;
-    ps->barg[n] = arena_of(blockIdx.x) + ((unsigned long long)q.off16 << 4) + HDR;
+    ps->barg[n] = arena_of(blockIdx.x) + off + HDR;
     ps->bstash[n] = j;
     ps->bkeys[n] = key;
     ps->nb = n + 1;
@@ -1442,7 +1458,7 @@ __device__ void next_action() {
         break;
       }
       stash_key* k = keys_of(slot) + (i % S);
-      // from the list's record, on chip; with an overflowed list from the key
+      // from the list's record, on chip; without one from the key
       const ready_rec* q = rec >= 0 ? &ps->rq_rec[rec] : nullptr;
       const int cid = q ? q->cid : k->chare_id, idx = q ? q->idx : k->chare_idx;
       chare_proxy_base* p = proxy_of(ps, cid);
@@ -1472,7 +1488,7 @@ __device__ void next_action() {
       ps->d_arg = env + HDR;
       ps->d_key = i;
       // (from the on-chip ready list; past RQ_MAX ready ones, one at a time)
-      if (p->warp_em(ep) && batching() && q) stash_batch(p, cid, idx, ep, ps->d_arg, i);
+      if (p->warp_em(ep) && batching() && !ps->rq_over) stash_batch(p, cid, idx, ep, ps->d_arg, i);
       return;
     }
     if (ps->revive_pending) continue;

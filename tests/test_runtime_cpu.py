@@ -215,6 +215,17 @@ def test_inline_entry_methods(emus, exe, n_pes, threads, n, m, refs):
     assert h["warp"] == n * (m // 3)
 
 
+@pytest.mark.parametrize("g", [30, 32, 34, 50, 62, 64, 66])
+def test_ready_messages_in_warp_batches(emus, g):
+    """4 * g messages to 4 chares in turn become ready at once, refnum after refnum:
+    all of them run in batches as long as the ready list holds them (256),
+    with a record on chip (128) or without; a longer list is taken one at a
+    time from the keys. The order is the same."""
+    h = ladder(emus["rt_emu_mt"], 1, 128, 4, 4 * g, 4, 1)
+    assert h["status"] == 0 and h["done"] == 4
+    assert h["batched"] == 16 * g if g <= 64 else 0 < h["batched"] < 16 * g
+
+
 @pytest.mark.parametrize("kind", [2, 3])
 @pytest.mark.parametrize("exe,threads", [("rt_emu", 1), ("rt_emu_mt", 64)])
 def test_inline_entry_method_returning_no_block_entry_method(emus, exe, threads, kind):
