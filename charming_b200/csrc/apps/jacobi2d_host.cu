@@ -64,28 +64,44 @@ __device__ __forceinline__ T* cell(const jac::chare_desc& d, int b, int r, int c
 }
 
 // The three kernels below move whole grids between chare blocks and a
-// problem's global grid (or bc) and are bound by HBM: blocks of 64 x 4
-// threads, blockIdx.x the chare, its rows dealt over blockIdx.y and the 4
-// thread rows, no division per cell. With one block per chare (or a division
-// or four per cell) an 8192^2 load or store spent 0.9 and 0.3 ms in them.
-constexpr int GRID_TX = 64, GRID_TY = 4;
+// problem's global grid (or bc) and are bound by HBM, or by latency on small
+// grids. init and scatter: blocks of tx x ty threads, blockIdx.x the chare, its
+// rows dealt over blockIdx.y and the ty thread rows, its columns over blockIdx.z
+// and tx, no division per cell. With one block per chare (or a division or four
+// per cell) an 8192^2 load or store spent 0.9 and 0.3 ms in them.
+struct grid_shape {
+  dim3 blocks, threads;
+};
+// For chares of at most rows x cols cells: no more threads than a chare has
+// cells for, and about 4096 blocks of them whatever the number of chares, as
+// far as the cells go. (64 x 4 threads and at most 64 blocks for a chare: load
+// of one 200000 x 16 FP64 chare 1.6 ms, 0.56 this way.)
+grid_shape shape_for(int chares, int rows, int cols) {
+  int tx = 64, ty = 1;
+  while (tx > 8 && tx / 2 >= cols) tx /= 2;
+  while (tx * ty < 256 && ty < rows) ty *= 2;
+  const int budget = std::max(1, 4096 / chares);
+  const int gy = std::min(budget, (rows + ty - 1) / ty);
+  const int gz = std::max(1, std::min(budget / gy, (cols + 4 * tx - 1) / (4 * tx)));
+  return grid_shape{dim3((unsigned)chares, (unsigned)gy, (unsigned)gz), dim3((unsigned)tx, (unsigned)ty)};
+}
 
 // Initial state: boundary ring from bc (top/bottom rows include the corners),
 // interior 0; written to both buffers over the whole ghost zone wherever the
 // position lies on the global grid (ghost cells on the domain boundary must
 // hold boundary values for the multi-sweep pass).
 template <typename T>
-__global__ void __launch_bounds__(GRID_TX * GRID_TY) init_kernel(const jac::chare_desc* ch, const jac::prob_desc* pr,
+__global__ void __launch_bounds__(256) init_kernel(const jac::chare_desc* ch, const jac::prob_desc* pr,
     const double* bc) {
   const jac::chare_desc& d = ch[blockIdx.x];
   const jac::prob_desc& p = pr[d.prob];
   const double* b = bc + 4 * d.prob;
   const int D = d.depth, nx = p.nx, ny = p.ny;
-  for (int r = 1 - D + (int)(blockIdx.y * GRID_TY + threadIdx.y); r <= d.h + D; r += (int)(gridDim.y * GRID_TY)) {
+  for (int r = 1 - D + (int)(blockIdx.y * blockDim.y + threadIdx.y); r <= d.h + D; r += (int)(gridDim.y * blockDim.y)) {
     const int gy = d.y0 + r;
     if (gy < 0 || gy > ny + 1) continue;
     T *a0 = cell<T>(d, 0, r, 0), *a1 = cell<T>(d, 1, r, 0);
-    for (int c = 1 - D + (int)threadIdx.x; c <= d.w + D; c += GRID_TX) {
+    for (int c = 1 - D + (int)(blockIdx.z * blockDim.x + threadIdx.x); c <= d.w + D; c += (int)(gridDim.z * blockDim.x)) {
       const int gx = d.x0 + c;
       if (gx < 0 || gx > nx + 1) continue;
       const double v = gy == 0 ? b[0] : gy == ny + 1 ? b[1] : gx == 0 ? b[2] : gx == nx + 1 ? b[3] : 0.0;
@@ -97,42 +113,44 @@ __global__ void __launch_bounds__(GRID_TX * GRID_TY) init_kernel(const jac::char
 // Global grid (ny+2) x (nx+2) in `stage` -> blocks of one problem (whole
 // ghost zone, as init_kernel).
 template <typename T>
-__global__ void __launch_bounds__(GRID_TX * GRID_TY) scatter_kernel(const jac::chare_desc* ch, const int* chare_of,
+__global__ void __launch_bounds__(256) scatter_kernel(const jac::chare_desc* ch, const int* chare_of,
     int nx, int ny, const T* stage) {
   const jac::chare_desc& d = ch[chare_of[blockIdx.x]];
   const int D = d.depth;
-  for (int r = 1 - D + (int)(blockIdx.y * GRID_TY + threadIdx.y); r <= d.h + D; r += (int)(gridDim.y * GRID_TY)) {
+  for (int r = 1 - D + (int)(blockIdx.y * blockDim.y + threadIdx.y); r <= d.h + D; r += (int)(gridDim.y * blockDim.y)) {
     const int gy = d.y0 + r;
     if (gy < 0 || gy > ny + 1) continue;
     T *__restrict__ a0 = cell<T>(d, 0, r, 0), *__restrict__ a1 = cell<T>(d, 1, r, 0);
     const T* __restrict__ src = stage + (size_t)gy * (nx + 2) + d.x0;
     const int c0 = max(1 - D, -d.x0), c1 = min(d.w + D, nx + 1 - d.x0);
 #pragma unroll 4
-    for (int c = c0 + (int)threadIdx.x; c <= c1; c += GRID_TX) a0[c] = a1[c] = src[c];
+    for (int c = c0 + (int)(blockIdx.z * blockDim.x + threadIdx.x); c <= c1; c += (int)(gridDim.z * blockDim.x)) a0[c] = a1[c] = src[c];
   }
 }
 
 // Blocks of one problem -> global grid: interior cells from their owner,
-// ring cells from the ghost ring of the edge chare next to them.
+// ring cells from the ghost ring of the edge chare next to them. A block takes
+// one row of chares and blockDim.x columns of the grid, whatever chares these
+// lie in, so that rows of small chares are stored together too. Calls of store,
+// us, with a block per chare as in scatter / this way (a thread per cell with
+// two divisions): FP32 200000 x 16 in one chare 772 / 278 (294), 8192^2 in one
+// chare 6577 / 4872 (5151), FP64 2048^2 in 8 x 8 chares 740 / 642 (665).
 template <typename T>
-__global__ void __launch_bounds__(GRID_TX * GRID_TY) gather_kernel(const jac::chare_desc* ch, const int* chare_of,
-    const int* final_buf, int nx, int ny, int px, int py, T* stage) {
-  const int k = chare_of[blockIdx.x];
+__global__ void __launch_bounds__(256) gather_kernel(const jac::chare_desc* ch, const int* chare_of,
+    const int* final_buf, int nx, int ny, int px, int py, int col_blocks, T* stage) {
+  const int cy = (int)blockIdx.x / col_blocks;
+  const int gx = ((int)blockIdx.x - cy * col_blocks) * (int)blockDim.x + (int)threadIdx.x;
+  if (gx > nx + 1) return;
+  const int k = chare_of[cy * px + jac::split_owner(nx, px, min(max(gx - 1, 0), nx - 1))];
   const jac::chare_desc& d = ch[k];
-  const int fb = final_buf[k];
-  const int r0 = d.cy == 0 ? 0 : 1, r1 = d.cy == py - 1 ? d.h + 1 : d.h;
-  const int c0 = d.cx == 0 ? 0 : 1, c1 = d.cx == px - 1 ? d.w + 1 : d.w;
-  for (int r = r0 + (int)(blockIdx.y * GRID_TY + threadIdx.y); r <= r1; r += (int)(gridDim.y * GRID_TY)) {
-    const T* __restrict__ src = cell<T>(d, fb, r, 0);
-    T* __restrict__ dst = stage + (size_t)(d.y0 + r) * (nx + 2) + d.x0;
+  const int r0 = cy == 0 ? 0 : 1, r1 = cy == py - 1 ? d.h + 1 : d.h;
+  const T* __restrict__ src = cell<T>(d, final_buf[k], 0, gx - d.x0);
+  const size_t sp = (size_t)d.pitch, dp = (size_t)nx + 2;
+  T* __restrict__ dst = stage + (size_t)d.y0 * dp + gx;
 #pragma unroll 4
-    for (int c = c0 + (int)threadIdx.x; c <= c1; c += GRID_TX) dst[c] = src[c];
-  }
+  for (int r = r0 + (int)(blockIdx.y * blockDim.y + threadIdx.y); r <= r1; r += (int)(gridDim.y * blockDim.y))
+    dst[r * dp] = src[r * sp];
 }
-
-// Enough blocks for a few waves whatever the number of chares.
-dim3 grid_blocks(int chares) { return dim3((unsigned)chares, (unsigned)std::min(64, std::max(1, 4096 / chares))); }
-constexpr dim3 grid_threads() { return dim3(GRID_TX, GRID_TY); }
 
 int fail(int code, const char* msg) {
   charm_host::set_error_text(msg);
@@ -140,6 +158,14 @@ int fail(int code, const char* msg) {
 }
 
 int check_cuda(cudaError_t e, const char* what) { return charm_host::cuda_fail(e, what); }
+
+// The shape for problem prob's chares and `ghost` rows and columns around them.
+grid_shape shape_of(const JHandle* h, int prob, int ghost) {
+  const charming_jacobi_problem& q = h->probs[prob];
+  const int px = h->px[prob], py = h->py[prob];
+  return shape_for(px * py, (q.ny + py - 1) / py + 2 * ghost, (q.nx + px - 1) / px + 2 * ghost);
+}
+int depth_of(const JHandle* h, int prob) { return h->chares[(size_t)h->chare_of[h->chare_of_off[prob]]].depth; }
 
 }  // namespace
 
@@ -268,8 +294,14 @@ extern "C" int charming_jacobi2d_init(void* handle) {
   JHandle* h = reinterpret_cast<JHandle*>(handle);
   if (!h) return CHARMING_ERR_CONFIG;
   cudaStream_t s = charm_host::stream();
-  if (h->esz == 8) init_kernel<double><<<grid_blocks(h->n_chares), grid_threads(), 0, s>>>(h->d_chares, h->d_probs, h->d_bc);
-  else init_kernel<float><<<grid_blocks(h->n_chares), grid_threads(), 0, s>>>(h->d_chares, h->d_probs, h->d_bc);
+  int rows = 1, cols = 1;
+  for (const jac::chare_desc& d : h->chares) {
+    rows = std::max(rows, d.h + 2 * d.depth);
+    cols = std::max(cols, d.w + 2 * d.depth);
+  }
+  const grid_shape g = shape_for(h->n_chares, rows, cols);
+  if (h->esz == 8) init_kernel<double><<<g.blocks, g.threads, 0, s>>>(h->d_chares, h->d_probs, h->d_bc);
+  else init_kernel<float><<<g.blocks, g.threads, 0, s>>>(h->d_chares, h->d_probs, h->d_bc);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemsetAsync(h->d_final, 0, sizeof(int) * h->n_chares, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -280,21 +312,26 @@ extern "C" int charming_jacobi2d_init(void* handle) {
 // blocks -> staged grid) on stream s, without the host copies.
 static void enqueue_scatter(JHandle* h, int prob, const void* stage, cudaStream_t s) {
   const charming_jacobi_problem& q = h->probs[prob];
-  const dim3 g = grid_blocks(h->px[prob] * h->py[prob]), t = grid_threads();
+  const grid_shape g = shape_of(h, prob, depth_of(h, prob));
   const int* co = h->d_chare_of + h->chare_of_off[prob];
-  if (h->esz == 8) scatter_kernel<double><<<g, t, 0, s>>>(h->d_chares, co, q.nx, q.ny, (const double*)stage);
-  else scatter_kernel<float><<<g, t, 0, s>>>(h->d_chares, co, q.nx, q.ny, (const float*)stage);
+  if (h->esz == 8)
+    scatter_kernel<double><<<g.blocks, g.threads, 0, s>>>(h->d_chares, co, q.nx, q.ny, (const double*)stage);
+  else
+    scatter_kernel<float><<<g.blocks, g.threads, 0, s>>>(h->d_chares, co, q.nx, q.ny, (const float*)stage);
 }
 static void enqueue_gather(JHandle* h, int prob, void* stage, cudaStream_t s) {
   const charming_jacobi_problem& q = h->probs[prob];
-  const dim3 g = grid_blocks(h->px[prob] * h->py[prob]), t = grid_threads();
+  const int px = h->px[prob], py = h->py[prob], rows = (q.ny + py - 1) / py + 2;
+  int tx = 64, ty = 1;
+  while (tx > 8 && tx / 2 >= q.nx + 2) tx /= 2;
+  while (tx * ty < 256 && ty < rows) ty *= 2;
+  const int col_blocks = (q.nx + 2 + tx - 1) / tx, n = col_blocks * py;
+  const dim3 g((unsigned)n, (unsigned)std::max(1, std::min(4096 / n, (rows + ty - 1) / ty))), t(tx, ty);
   const int* co = h->d_chare_of + h->chare_of_off[prob];
   if (h->esz == 8)
-    gather_kernel<double><<<g, t, 0, s>>>(h->d_chares, co, h->d_final, q.nx, q.ny, h->px[prob], h->py[prob],
-                                          (double*)stage);
+    gather_kernel<double><<<g, t, 0, s>>>(h->d_chares, co, h->d_final, q.nx, q.ny, px, py, col_blocks, (double*)stage);
   else
-    gather_kernel<float><<<g, t, 0, s>>>(h->d_chares, co, h->d_final, q.nx, q.ny, h->px[prob], h->py[prob],
-                                         (float*)stage);
+    gather_kernel<float><<<g, t, 0, s>>>(h->d_chares, co, h->d_final, q.nx, q.ny, px, py, col_blocks, (float*)stage);
 }
 
 static int ensure_stage(JHandle* h, size_t bytes) {
