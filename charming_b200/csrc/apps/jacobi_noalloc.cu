@@ -70,6 +70,11 @@ int scratch_on_current_device(void** out, int* sms) {
 // boundary ring included (it is copied), with the chares' wavefront
 // (jac::deep_step): a warp streams the rows of one item, a strip of 32
 // vectors times a run of rows, and keeps the levels between in registers.
+// Grids of at most 16 vectors a row need no strips: a warp takes 32 / G items
+// of G lanes, each a whole row wide (the boundary columns at both ends are kept
+// at every level, so what the shuffles bring from the next item is not used).
+// 1 x 690000 FP32, 20 sweeps: 98 us; 1033 in strips with most lanes idle, 144
+// with one launch per sweep.
 // Rows have any alignment here: ALIGNED (16-byte aligned grids whose rows are
 // whole vectors) loads and stores vectors, else element by element. The next
 // NA_U rows are in flight in registers. FIX: the item's levels can meet the
@@ -79,15 +84,17 @@ int scratch_on_current_device(void** out, int* sms) {
 // per point); 2046^2 FP32, 100 sweeps: 320 us (1870 so).
 constexpr int NA_U = 4;
 
+// v: the lane's vector, own: it stores it; rows r0 .. r1 - 1 (none if r1 <= r0)
+// in `run` + 2 L steps, the same number for all lanes of the warp.
 template <typename T, int L, bool ALIGNED, bool FIX>
 __device__ __forceinline__ void noalloc_item(const T* __restrict__ src, T* __restrict__ dst, int nx, int ny,
-    int own0, int nown, int r0, int r1) {
-  constexpr int V = jac::traits<T>::VEC, E = (L + V - 1) / V, LH = (L + 1) / 2, U = NA_U;
-  const int lane = (int)(threadIdx.x & 31), v = own0 - E + lane, col0 = v * V, W = nx + 2;
+    int v, bool own, int r0, int r1, int run) {
+  constexpr int V = jac::traits<T>::VEC, LH = (L + 1) / 2, U = NA_U;
+  const int col0 = v * V, W = nx + 2;
   jac::deep_lane<T> ln;
   ln.v = v;
   ln.col0 = col0;
-  ln.own = lane >= E && lane < E + nown;
+  ln.own = own;
   ln.anyfix = false;
 #pragma unroll
   for (int k = 0; k < V; k++) {
@@ -96,7 +103,7 @@ __device__ __forceinline__ void noalloc_item(const T* __restrict__ src, T* __res
   }
   ln.fix_r0 = 0;
   ln.fix_r1 = ny + 1;
-  const int qs = r0 - L, qe = r1 - 1 + L;
+  const int qs = r0 - L, qe = r1 - 1 + L, qend = r0 + run - 1 + L;
   // columns and rows off the grid: its nearest ones, never used by a result
   int off[V];
 #pragma unroll
@@ -141,7 +148,7 @@ __device__ __forceinline__ void noalloc_item(const T* __restrict__ src, T* __res
     }
   }
 #pragma unroll 1
-  for (; q <= qe; q += U) {
+  for (; q <= qend; q += U) {
 #pragma unroll
     for (int u = 0; u < U; u++) {
 #pragma unroll
@@ -164,15 +171,22 @@ __device__ __forceinline__ void noalloc_item(const T* __restrict__ src, T* __res
 
 template <typename T, int L, bool ALIGNED>
 __global__ void __launch_bounds__(128) noalloc_pass_kernel(const T* __restrict__ src, T* __restrict__ dst, int nx,
-    int ny, int strips, int run_rows, int items) {
+    int ny, int strips, int group, int run_rows, int warps) {
   constexpr int V = jac::traits<T>::VEC, E = (L + V - 1) / V, SS = 32 - 2 * E;
-  const int item = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (item >= items) return;
-  const int nv = (nx + 2 + V - 1) / V, own0 = item % strips * SS, nown = min(SS, nv - own0);
-  const int r0 = item / strips * run_rows, r1 = min(ny + 2, r0 + run_rows);
+  const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = (int)(threadIdx.x & 31);
+  if (w >= warps) return;
+  const int nv = (nx + 2 + V - 1) / V;
+  if (group < 32) {
+    const int v = lane & (group - 1), r0 = (w * (32 / group) + lane / group) * run_rows;
+    noalloc_item<T, L, ALIGNED, true>(src, dst, nx, ny, v, v < nv, r0, min(ny + 2, r0 + run_rows), run_rows);
+    return;
+  }
+  const int own0 = w % strips * SS, nown = min(SS, nv - own0), v = own0 - E + lane;
+  const bool own = lane >= E && lane < E + nown;
+  const int r0 = w / strips * run_rows, r1 = min(ny + 2, r0 + run_rows);
   const bool edge = own0 - E <= 0 || (own0 + nown + E) * V > nx + 1 || r0 - L <= 0 || r1 - 1 + L >= ny + 1;
-  if (edge) noalloc_item<T, L, ALIGNED, true>(src, dst, nx, ny, own0, nown, r0, r1);
-  else noalloc_item<T, L, ALIGNED, false>(src, dst, nx, ny, own0, nown, r0, r1);
+  if (edge) noalloc_item<T, L, ALIGNED, true>(src, dst, nx, ny, v, own, r0, r1, r1 - r0);
+  else noalloc_item<T, L, ALIGNED, false>(src, dst, nx, ny, v, own, r0, r1, r1 - r0);
 }
 
 constexpr int NA_LMAX = 8;
@@ -181,22 +195,27 @@ constexpr int NA_LMAX = 8;
 // pass costs its launch and first loads (5000), then its rows: a warp's step
 // through one level takes 55 cycles alone and 38 of its SM sub-partition's
 // when several warps share it. (Measured on a B200 to within a quarter; the
-// choice only needs their ratio.)
+// choice only needs their ratio.) Chosen on every call, 8 lengths times about
+// 20 splits, so with few divisions.
 struct pass_plan {
-  int run_rows, strips, items;
+  int run_rows, strips, group, warps;
   double cycles;
 };
 template <typename T>
 pass_plan plan_pass(int L, int nx, int ny, int sms) {
   constexpr int V = jac::traits<T>::VEC;
-  const int E = (L + V - 1) / V, SS = 32 - 2 * E, rows = ny + 2;
-  const int strips = ((nx + 2 + V - 1) / V + SS - 1) / SS;
-  pass_plan best{0, strips, 0, 1e300};
+  const int E = (L + V - 1) / V, SS = 32 - 2 * E, rows = ny + 2, nv = (nx + 2 + V - 1) / V;
+  int group = 32, sh = 0;  // 1 << sh items a warp
+  for (; group > 1 && group / 2 >= nv; group /= 2) sh++;
+  const int strips = group < 32 ? 1 : (nv + SS - 1) / SS;
+  const double inv_parts = 1.0 / (4.0 * sms);
+  pass_plan best{0, strips, group, 0, 1e300};
   for (int R = 4; R <= 128; R += R < 16 ? 2 : R < 64 ? 8 : 32) {
     const long long items = (long long)strips * ((rows + R - 1) / R);
-    const double per_part = std::ceil((double)items / (4.0 * sms));
+    const long long warps = (items + (1 << sh) - 1) >> sh;
+    const double per_part = std::ceil((double)warps * inv_parts);
     const double c = 5000.0 + (double)(std::min(R, rows) + 2 * L) * L * std::max(55.0, 38.0 * per_part);
-    if (c < best.cycles) best = pass_plan{R, strips, (int)items, c};
+    if (c < best.cycles) best = pass_plan{R, strips, group, (int)warps, c};
     if (R >= rows) break;
   }
   return best;
@@ -204,11 +223,11 @@ pass_plan plan_pass(int L, int nx, int ny, int sms) {
 
 template <typename T, int L>
 void launch_pass(const T* src, T* dst, int nx, int ny, const pass_plan& p, bool aligned, int sms) {
-  // few items: blocks of one warp, so that they spread over the SMs
-  const int threads = p.items <= 4 * sms ? 32 : p.items <= 8 * sms ? 64 : 128;
-  const int blocks = (int)(((long long)p.items * 32 + threads - 1) / threads);
-  if (aligned) noalloc_pass_kernel<T, L, true><<<blocks, threads, 0, 0>>>(src, dst, nx, ny, p.strips, p.run_rows, p.items);
-  else noalloc_pass_kernel<T, L, false><<<blocks, threads, 0, 0>>>(src, dst, nx, ny, p.strips, p.run_rows, p.items);
+  // few warps: blocks of one warp, so that they spread over the SMs
+  const int threads = p.warps <= 4 * sms ? 32 : p.warps <= 8 * sms ? 64 : 128;
+  const int blocks = (int)(((long long)p.warps * 32 + threads - 1) / threads);
+  auto fn = aligned ? noalloc_pass_kernel<T, L, true> : noalloc_pass_kernel<T, L, false>;
+  fn<<<blocks, threads, 0, 0>>>(src, dst, nx, ny, p.strips, p.group, p.run_rows, p.warps);
 }
 template <typename T>
 void launch_pass_of(int L, const T* src, T* dst, int nx, int ny, const pass_plan& p, bool aligned, int sms) {

@@ -83,6 +83,10 @@ def test_put_halos_units(rt, dtype, depth):
 @pytest.mark.parametrize("nx,ny,sweeps,shift", [
     (1, 1, 3, 0), (2, 5, 1, 0), (3, 2, 9, 1), (6, 300, 7, 0), (301, 4, 8, 0), (46, 33, 2, 1), (54, 61, 13, 0),
     (110, 130, 17, 0), (111, 97, 23, 1), (510, 254, 20, 0), (1022, 1020, 11, 0), (1445, 1441, 10, 1),
+    # rows of at most 16 vectors: groups of 1 to 16 lanes (2, 4, 8, 16 and 32
+    # items a warp), the widest of each type, and the next wider grid in strips
+    (1, 5000, 8, 0), (2, 777, 5, 1), (4, 4001, 8, 0), (6, 33, 3, 0), (12, 2503, 20, 1), (14, 900, 7, 0),
+    (28, 129, 6, 0), (30, 1000, 16, 0), (31, 1000, 8, 0), (61, 700, 9, 1), (62, 701, 8, 0), (63, 702, 8, 0),
 ])
 def test_noalloc_pass_edges(rt, dtype, nx, ny, sweeps, shift):
     torch = pytest.importorskip("torch")
