@@ -45,23 +45,33 @@ struct j3_geom {
 // level and step parity
 constexpr size_t j3_smem(int warps, int L, int RY) { return (size_t)warps * 512 * (J3_S * RY + 4 * L); }
 
+// Grids of at most 16 vectors a row need no strips: a warp takes the rows of
+// 32 >> gs groups of 1 << gs lanes, each a whole row wide (the shell columns at
+// both ends are kept at every level, so what the shuffles bring from the next
+// group is not used). gs 5: whole warps. 1 x 1 x 300000, 3 sweeps: 154 us (1790
+// in strips of whole warps and at most 64 runs, 1279 with one sweep per pass),
+// 1 x 200000 x 4 51 (960, 392), 20 x 3000 x 100, 6 sweeps 135 (260, 355).
 struct j3_plan {
-  int warps, yown, yblocks, zrun, zruns, strips;
+  int warps, gs, yown, yblocks, zrun, zruns, strips;
   double cost;
 };
 
-template <int L, int RY, bool FIX>
+// GRP: groups of fewer lanes than a warp's (compiled apart: in one kernel with
+// them wide grids took 4 to 10 % longer).
+template <int L, int RY, bool FIX, bool GRP>
 __device__ __forceinline__ void j3_tile(const double* __restrict__ in, double* __restrict__ out, int nx, int ny,
-    int nz, int pitch, int zrun, int yown, double2* smem) {
+    int nz, int pitch, int zrun, int yown, int gs, double2* smem) {
   using G = j3_geom<L>;
   constexpr unsigned FULL = 0xffffffffu;
-  const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
-  const int NT = (int)blockDim.x, W = nx + 2;
+  // lane, group of lanes (a warp) and groups; GW lanes lie between two groups
+  const int GS = GRP ? gs : 5, GW = 1 << GS, lane = (int)threadIdx.x & (GW - 1), grp = (int)threadIdx.x >> GS;
+  const int ngrp = (int)blockDim.x >> GS, NT = (int)blockDim.x, W = nx + 2;
   const size_t plane = (size_t)pitch * (ny + 2);
-  const int own0 = (int)blockIdx.x * G::SS, col0 = (own0 - G::E + lane) * 2;
+  constexpr int E = GRP ? 0 : G::E;
+  const int own0 = (int)blockIdx.x * G::SS, col0 = (own0 - E + lane) * 2;
   const int nv = (W + 1) / 2;
-  const bool own = lane >= G::E && lane < G::E + min(G::SS, nv - own0);
-  const int y0 = (int)blockIdx.y * yown, yt = y0 - L + warp * RY;  // the warp's first row
+  const bool own = lane >= E && lane < E + min(GRP ? GW : G::SS, nv - own0);
+  const int y0 = (int)blockIdx.y * yown, yt = y0 - L + grp * RY;  // the group's first row
   const int z0 = (int)blockIdx.z * zrun, z1 = min(nz + 2, z0 + zrun);
   const int qs = z0 - L, qe = z1 - 1 + L;
   const bool fixc0 = col0 == 0 || col0 == nx + 1, fixc1 = col0 + 1 == nx + 1;
@@ -135,13 +145,13 @@ __device__ __forceinline__ void j3_tile(const double* __restrict__ in, double* _
       const double t[2] = {v[L][i].x, v[L][i].y};
       jac::put_vec(p, t, n);
     }
-    __syncthreads();  // the edge rows of every warp and level are there
+    __syncthreads();  // the edge rows of every group and level are there
 #pragma unroll
     for (int l = 0; l < L; l++) {
-      // the rows above and below the warp's (at the block's edge: its own,
+      // the rows above and below the group's (at the block's edge: its own,
       // never used by a result)
-      const double2 up = e[(2 * l + 1) * NT - (warp > 0 ? 32 : 0)];
-      const double2 dn = e[(2 * l) * NT + (warp + 1 < nw ? 32 : 0)];
+      const double2 up = e[(2 * l + 1) * NT - (grp > 0 ? GW : 0)];
+      const double2 dn = e[(2 * l) * NT + (grp + 1 < ngrp ? GW : 0)];
 #pragma unroll
       for (int i = 0; i < RY; i++) {
         const double2 c = v[l][i];
@@ -157,45 +167,51 @@ __device__ __forceinline__ void j3_tile(const double* __restrict__ in, double* _
   jac::cp_async_wait<0>();
 }
 
-template <int L, int RY>
+template <int L, int RY, bool GRP>
 __global__ void __launch_bounds__(32 * J3_NWMAX, 1) jacobi3d_pass_kernel(const double* __restrict__ in,
-    double* __restrict__ out, int nx, int ny, int nz, int pitch, int zrun, int yown) {
+    double* __restrict__ out, int nx, int ny, int nz, int pitch, int zrun, int yown, int gs) {
   extern __shared__ __align__(16) double2 j3_shared[];
   using G = j3_geom<L>;
   const int own0 = (int)blockIdx.x * G::SS, y0 = (int)blockIdx.y * yown, z0 = (int)blockIdx.z * zrun;
   // the tile's levels can meet the shell
-  const bool edge = own0 - G::E <= 0 || (own0 + G::SS + G::E) * 2 > nx + 1 || y0 - L <= 0 ||
+  const bool edge = GRP || own0 - G::E <= 0 || (own0 + G::SS + G::E) * 2 > nx + 1 || y0 - L <= 0 ||
                     y0 - L + (int)(blockDim.x >> 5) * RY > ny + 1 || z0 - L <= 0 || z0 + zrun + L > nz + 1;
-  if (edge) j3_tile<L, RY, true>(in, out, nx, ny, nz, pitch, zrun, yown, j3_shared);
-  else j3_tile<L, RY, false>(in, out, nx, ny, nz, pitch, zrun, yown, j3_shared);
+  if (edge) j3_tile<L, RY, true, GRP>(in, out, nx, ny, nz, pitch, zrun, yown, gs, j3_shared);
+  else j3_tile<L, RY, false, false>(in, out, nx, ny, nz, pitch, zrun, yown, gs, j3_shared);
 }
 
 // Warps per block, rows per block and planes per run: the fewest steps of
 // all resident warps, over the waves that the launch takes. A block's rows
-// are its warps' less the 2L of the overlap, a run streams 2L planes more
+// are its groups' less the 2L of the overlap, a run streams 2L planes more
 // than it writes; with few blocks the warps of an SM are bound by latency
-// (taken as 8 warps' worth of time).
+// (taken as 8 warps' worth of time). Groups of few lanes make short runs of
+// many blocks cheap, so there the three steps that a run takes to start count
+// too (in the choice for wide grids they cost 256^3 17 %).
 template <int L, int RY>
 j3_plan j3_choose(int nx, int ny, int nz, int n_sms) {
-  const int strips = ((nx + 2 + 1) / 2 + j3_geom<L>::SS - 1) / j3_geom<L>::SS;
+  const int nv = (nx + 2 + 1) / 2;
+  int gs = 5;
+  while (gs > 1 && (1 << (gs - 1)) >= nv) gs--;
+  const int start = gs < 5 ? 3 : 0, strips = gs < 5 ? 1 : (nv + j3_geom<L>::SS - 1) / j3_geom<L>::SS;
   j3_plan best{};
   best.cost = 1e300;
-  for (int nw = (2 * L + RY) / RY; nw <= J3_NWMAX; nw++) {
-    const int ymax = nw * RY - 2 * L;
+  for (int nw = 1; nw <= J3_NWMAX; nw++) {
+    const int ymax = (nw * 32 >> gs) * RY - 2 * L;
     if (ymax < 1) continue;
     const int yb = (ny + 2 + ymax - 1) / ymax;
     if (yb > 65535 && nw < J3_NWMAX) continue;  // grid limit
     const int yown = (ny + 2 + yb - 1) / yb;
     const int per_sm = std::max(1, std::min(J3_NWMAX / nw, (int)((227u << 10) / (j3_smem(nw, L, RY) + 1024))));
     const long long tiles = (long long)strips * yb;
-    for (int runs = 1; runs <= 64; runs++) {
+    // (past 64 runs in steps of an eighth: tall grids of few rows)
+    for (int runs = 1; runs <= 16384; runs += runs < 64 ? 1 : runs / 8) {
       const int zr = (nz + 2 + runs - 1) / runs;
       if (runs > 1 && zr < 4 * L) break;
       const long long blocks = tiles * ((nz + 2 + zr - 1) / zr);
       const double waves = std::ceil((double)blocks / ((double)n_sms * per_sm));
       const double resident = std::min<double>(per_sm, std::ceil((double)blocks / n_sms));
-      const double cost = waves * (zr + 2 * L) * std::max(8.0, resident * nw) * RY / L;
-      if (cost < best.cost * 0.999) best = j3_plan{nw, yown, yb, zr, (nz + 2 + zr - 1) / zr, strips, cost};
+      const double cost = waves * (zr + 2 * L + start) * std::max(8.0, resident * nw) * RY / L;
+      if (cost < best.cost * 0.999) best = j3_plan{nw, gs, yown, yb, zr, (nz + 2 + zr - 1) / zr, strips, cost};
       if (zr == 1) break;
     }
   }
@@ -205,12 +221,12 @@ j3_plan j3_choose(int nx, int ny, int nz, int n_sms) {
 template <int L, int RY>
 cudaError_t j3_pass(const double* in, double* out, int nx, int ny, int nz, int pitch, const j3_plan& p,
     cudaStream_t s) {
-  auto fn = jacobi3d_pass_kernel<L, RY>;
+  auto fn = p.gs < 5 ? jacobi3d_pass_kernel<L, RY, true> : jacobi3d_pass_kernel<L, RY, false>;
   const size_t smem = j3_smem(p.warps, L, RY);
   cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)j3_smem(J3_NWMAX, L, RY));
   if (e != cudaSuccess) return e;
-  fn<<<dim3(p.strips, p.yblocks, p.zruns), 32 * p.warps, smem, s>>>(in, out, nx, ny, nz, pitch, p.zrun, p.yown);
+  fn<<<dim3(p.strips, p.yblocks, p.zruns), 32 * p.warps, smem, s>>>(in, out, nx, ny, nz, pitch, p.zrun, p.yown, p.gs);
   return cudaGetLastError();
 }
 

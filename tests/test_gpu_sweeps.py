@@ -113,6 +113,9 @@ def test_noalloc_pass_edges(rt, dtype, nx, ny, sweeps, shift):
 @pytest.mark.parametrize("nx,ny,nz,sweeps", [
     (1, 1, 1, 3), (3, 2, 5, 4), (58, 44, 9, 2), (59, 45, 10, 3), (61, 46, 33, 1), (62, 5, 70, 6), (120, 100, 40, 4),
     (257, 31, 12, 5), (20, 300, 16, 2), (124, 90, 130, 7),
+    # rows of at most 16 vectors: groups of 2 to 16 lanes; more than 64 runs
+    (1, 400, 5, 4), (2, 3, 700, 6), (4, 97, 12, 3), (5, 41, 9, 2), (6, 200, 20, 7), (13, 500, 3, 6), (14, 9, 900, 3),
+    (29, 77, 33, 5), (30, 64, 20, 6), (31, 64, 20, 6),
 ])
 def test_jacobi3d_tile_edges(rt, nx, ny, nz, sweeps):
     g = np.random.default_rng(nx + ny + nz).random((nz + 2, ny + 2, nx + 2))
