@@ -308,7 +308,8 @@ int charming_jacobi2d_sweeps_noalloc(int dtype, int nx, int ny, int sweeps,
  * jacobi_kernel.cu:36-48, multiplied by its literal 0.142857): grid is the
  * host's (nz+2) x (ny+2) x (nx+2) doubles, x fastest, shell fixed; it
  * receives the result of `sweeps` sweeps. *out_ms: device time of the
- * sweeps (copies excluded). */
+ * sweeps (without the copies from and to the host; for odd nx with those
+ * between the grid's rows and rows on 16-byte boundaries). */
 int charming_jacobi3d(int nx, int ny, int nz, int sweeps, double* grid, double* out_ms);
 
 /* Jacobi2d over a 1-D row decomposition (examples/jacobi2d-decomp1d/

@@ -121,3 +121,31 @@ def test_jacobi3d_tile_edges(rt, nx, ny, nz, sweeps):
     g = np.random.default_rng(nx + ny + nz).random((nz + 2, ny + 2, nx + 2))
     out, _ms = rt.jacobi3d(g, sweeps)
     assert same_bits(out, oj.jacobi3d(g, sweeps))
+
+
+def test_jacobi3d_time_covers_the_row_copies(rt):
+    """Odd widths are copied to rows of whole vectors and back: the reported
+    device time has both copies in it (with no sweeps it is nothing but them).
+    Each reads and writes the grid, at no more than 20 TB/s (L2 included)."""
+    nx, ny, nz = 299, 300, 300
+    g = np.random.default_rng(1).random((nz + 2, ny + 2, nx + 2))
+    out, ms = rt.jacobi3d(g, 0)
+    assert same_bits(out, g)
+    assert ms > 4 * g.nbytes / 20e12 * 1e3
+
+
+# load and store of grids: narrow and wide ones, one chare and many, chares of
+# a few cells, columns beyond one block and chares that a block's columns share
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("nx,ny,px,py", [
+    (1, 1, 1, 1), (3, 700, 1, 1), (5, 300, 2, 7), (900, 2, 1, 1), (5000, 3, 9, 2), (62, 40, 3, 3), (63, 63, 63, 1),
+    (64, 64, 8, 8), (131, 77, 16, 11), (300, 260, 60, 65), (257, 1030, 1, 1), (4100, 300, 2, 1),
+])
+def test_load_store_round_trip(rt, dtype, nx, ny, px, py):
+    npdt = np.float64 if dtype == "f64" else np.float32
+    g = np.random.default_rng(nx * 3 + ny).random((ny + 2, nx + 2)).astype(npdt)
+    with Jacobi2D([Problem(nx, ny, 3, px=px, py=py)], dtype=dtype) as j:
+        j.load(0, g)
+        assert same_bits(j.store(0), g)
+        j.run()  # and from the other buffer
+        assert same_bits(j.store(0), oracle(g, 3))
