@@ -23,12 +23,14 @@
 // Bound by the load/store pipe (ring copies, edge rows, shuffles) and, on
 // small grids, by the chain of a plane's step. GLUP/s against one sweep per
 // pass (32 x 16 tiles, planes by cp.async): 256^3 399 (255), 512^3 507 (290),
-// 640^3 580 (293), 128^3 220, 299 x 300 x 250 428 (232).
+// 640^3 578 (293), 128^3 219, 299 x 300 x 250 432 with its row copies over 300
+// sweeps (232).
 #include "suite.cuh"
 #ifndef CHARMING_HOST_EMULATION
 #include "jacobi_sweep.cuh"
 #include "../host.cuh"
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 namespace {
@@ -234,14 +236,45 @@ cudaError_t j3_pass(const double* in, double* out, int nx, int ny, int nz, int p
 // every row starts on a 16-byte boundary (element copies and stores made the
 // sweeps of a 255^3 grid 1.65 times as long); these copy them between, inside
 // the time that the call reports.
+// A block takes a run of rows, its threads every 256th cell of them, eight in
+// flight; a thread's next cell is found by adding. Both ways for 299 x 300 x 250
+// 139 us (310 with a row per block), 33 x 300 x 3000 203 (428 with a row per
+// warp), 0.77 to 0.81 of the copy bandwidth.
 __global__ void __launch_bounds__(256) j3_repitch_kernel(const double* __restrict__ src, double* __restrict__ dst,
-    int W, int sp, int dp, long long rows) {
-  for (long long r = (long long)blockIdx.x; r < rows; r += (long long)gridDim.x)
-    for (int c = (int)threadIdx.x; c < W; c += 256) dst[r * dp + c] = src[r * sp + c];
+    int W, int sp, int dp, long long rows, int run) {
+  constexpr int B = 8;
+  const long long r0 = (long long)blockIdx.x * run;
+  const long long left = rows - r0;
+  const int nr = (int)(left < run ? left : run), dr = 256 / W, dc = 256 - dr * W;
+  src += r0 * sp;
+  dst += r0 * dp;
+  int r = (int)threadIdx.x / W, c = (int)threadIdx.x - r * W;
+  while (r < nr) {
+    double v[B];
+    long long off[B];
+    bool in[B];
+#pragma unroll
+    for (int k = 0; k < B; k++) {
+      in[k] = r < nr;
+      if (in[k]) v[k] = src[(long long)r * sp + c];
+      off[k] = (long long)r * dp + c;
+      r += dr;
+      c += dc;
+      if (c >= W) {
+        c -= W;
+        r++;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < B; k++)
+      if (in[k]) dst[off[k]] = v[k];
+  }
 }
 cudaError_t j3_repitch(const double* src, double* dst, int W, int sp, int dp, long long rows,
     cudaStream_t s) {
-  j3_repitch_kernel<<<(unsigned)std::min<long long>(rows, 148 * 16), 256, 0, s>>>(src, dst, W, sp, dp, rows);
+  // runs of about 2048 cells, at most 2^31 - 1 of them
+  const long long run = std::max<long long>(std::max(1, 2048 / W), (rows + INT_MAX - 1) / INT_MAX);
+  j3_repitch_kernel<<<(unsigned)((rows + run - 1) / run), 256, 0, s>>>(src, dst, W, sp, dp, rows, (int)run);
   return cudaGetLastError();
 }
 
