@@ -146,7 +146,8 @@ __shared__ charm::chare_proxy<JBlock>* jproxy;
 // This PE's phase timers (ns: sweeps, halo sending, halo entry methods),
 // kept on chip and stored through to japp::pe_ns() after every update (a
 // store only: no read of global memory on the message path).
-// Slots: 0 sweeps, 1 halo sends (all of send_halos), 2 halo entry methods,
+// Slots: 0 sweeps, 1 halo sends (all of send_halos), 2 halo entry methods
+// (with halos put into the ghost zones: their notes),
 // 3 of the sends: up to the ring space taken, 4 of the sends: publishing,
 // 5 of the sends: up to the reservation call.
 constexpr int PE_NS_SLOTS = 8;
@@ -158,6 +159,12 @@ __device__ __forceinline__ unsigned long long pe_clock() { return (unsigned long
 __device__ __forceinline__ void add_pe_cyc(int k, unsigned long long cyc) {
   s_pe_ns[k] += cyc;
   japp::pe_ns()[PE_NS_SLOTS * blockIdx.x + k] = s_pe_ns[k];
+}
+// Notes only add to their timer; the sweep that follows the last ones of a
+// pass stores it.
+__device__ __forceinline__ void add_sweep_cyc(unsigned long long cyc) {
+  add_pe_cyc(0, cyc);
+  japp::pe_ns()[PE_NS_SLOTS * blockIdx.x + 2] = s_pe_ns[2];
 }
 __shared__ charm::chare_proxy<JServer>* sproxy;
 
@@ -229,7 +236,7 @@ __device__ double sweep_block(const jac::chare_desc& d, int cur, bool resid, int
                 : jac::sweep_direct<T, false>(in, out, d.w, d.h);
     __syncthreads();
   }
-  if (threadIdx.x == 0) add_pe_cyc(0, pe_clock() - t0);
+  if (threadIdx.x == 0) add_sweep_cyc(pe_clock() - t0);
   return resid ? suite::block_sum_f64(acc) : 0.0;
 }
 

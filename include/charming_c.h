@@ -243,7 +243,8 @@ typedef struct charming_jacobi_info {
   double sweep_ms_max;        /* last run: max over PEs of time in sweeps  */
   double sweep_ms_mean;       /* last run: mean over busy PEs              */
   double send_ms_mean;        /* last run: mean time packing/sending halos */
-  double halo_ms_mean;        /* last run: mean time in halo entry methods */
+  double halo_ms_mean;        /* last run: mean time in halo entry methods (default halo
+                               * mode: counting the notes of the halos put) */
   /* the next three: builds with -DCHARMING_PROFILE only (else 0) */
   double send_reserve_ms_mean;  /* of send_ms_mean: taking the ring space    */
   double send_publish_ms_mean;  /* of send_ms_mean: publishing the messages  */

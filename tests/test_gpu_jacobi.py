@@ -274,3 +274,14 @@ def test_solve_stream_matches_load_run_store(rt, use_graph):
         assert ms > 0
         for g, o in zip(grids, outs):
             assert np.array_equal(bits(o), bits(jac64(g, 23)))
+
+
+@pytest.mark.parametrize("halo_mode,depth", [(0, 0), (0, 1), (1, 2)])
+def test_phase_times(rt, halo_mode, depth):
+    """Each phase timer of a run with neighbours counts something, whatever
+    way its halos take, and no more than the run."""
+    with Jacobi2D([Problem(600, 500, 60, px=5, py=4)], halo_mode=halo_mode, depth=depth) as j:
+        j.run()
+        i = j.info()
+    for k in ("sweep_ms_mean", "send_ms_mean", "halo_ms_mean"):
+        assert 0 < i[k] < i["last_run_ms"], (k, i)
