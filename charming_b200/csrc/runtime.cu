@@ -94,6 +94,27 @@ __device__ void charm::detail::report_error(int code, int info0, int info1) {
   set_error(code, info0, info1);
 }
 
+// In the place of an entry method that the block cannot run.
+namespace {
+__device__ void em_none(chare_proxy_base* base, int idx, void* arg) {
+  if (threadIdx.x == 0) charm::detail::report_error(charm::detail::ERR_BAD_TARGET, base->id, idx);
+}
+}  // namespace
+
+__device__ void charm::detail::add_inline_em(chare_proxy_base* p, em_inline_fn fn) {
+  const int ep = p->em_count;
+  if (p->em_tab == nullptr || ep >= INLINE_EM_MAX) {
+    report_error(ERR_TOO_MANY_EMS, p->id, ep);
+    return;
+  }
+  if (p->inline_ems == 0)
+    for (int k = ep; k <= INLINE_EM_MAX; k++) p->em_tab[k] = &em_none;
+  p->em_cap = INLINE_EM_MAX;
+  p->inline_ems |= 1ULL << ep;
+  p->em_tab[INLINE_EM_MAX + 1 + ep] = reinterpret_cast<em_entry_fn>(fn);
+  p->em_count = ep + 1;
+}
+
 namespace {
 __device__ __forceinline__ unsigned char* smem_arena() {
   return reinterpret_cast<unsigned char*>(s_mem) + c_rt.smem_state_bytes;
@@ -1382,8 +1403,7 @@ __device__ void stash_batch(chare_proxy_base* p, int cid, int idx, int ep, void*
 
 // Thread 0: runs entry method *ep of chare idx here if it is an inline one.
 // True when the delivery ended with it; else *ep is the entry method that the
-// block has to run. A returned number that is no block or warp-level entry
-// method of the proxy is an error (it would be called through the table).
+// block has to run (one that is none reports that when it is called).
 __device__ bool inline_done(pe_state* ps, chare_proxy_base* p, int idx, int* ep, void* arg) {
   if (!p->inline_em(*ep)) return false;
   const long long c0 = clock64();
@@ -1393,11 +1413,7 @@ __device__ bool inline_done(pe_state* ps, chare_proxy_base* p, int idx, int* ep,
     if ((++ps->stats[ST_DELIVERED] & 15) == 0) stamp_progress(ps->my_pe);
     return true;
   }
-  if (!p->valid_target(idx, next) || p->inline_em(next)) {
-    set_error(CHARMING_ERR_BAD_TARGET, p->id, next);
-    return true;
-  }
-  *ep = next;
+  *ep = min(next, INLINE_EM_MAX);
   return false;
 }
 

@@ -16,6 +16,7 @@
 
 #define CHARE_TYPE_CNT_MAX 1024 // Maximum number of chare types per PE
 #define EM_CNT_MAX 128          // Maximum number of entry methods per chare type
+#define INLINE_EM_MAX 63        // ... of one that has inline entry methods
 #define ASYNC_WAIT_MAX 16       // Pending async_waits per chare array per PE
 #define MISMATCH_MAX 128        // Kept for source compatibility (stash is per PE)
 
@@ -104,12 +105,19 @@ struct chare_proxy_base {
   // warp runs each of their deliveries.
   unsigned long long warp_ems;
   // ... and those registered with add_inline_entry_method: run by the
-  // scheduler's deciding thread (their em_tab entry is an em_inline_fn).
+  // scheduler's deciding thread. A proxy with any has at most INLINE_EM_MAX
+  // entry methods: the function of inline entry method ep is entry
+  // INLINE_EM_MAX + 1 + ep of em_tab, and entry ep, like every unused one up
+  // to INLINE_EM_MAX, reports an error, so that the number that an inline
+  // entry method returns is only cut to INLINE_EM_MAX (a check with its error
+  // in the scheduler's loop cost small chares 2 to 4 %).
   unsigned long long inline_ems;
+  int em_cap;    // how many fit: EM_CNT_MAX, or INLINE_EM_MAX
 
   __device__ chare_proxy_base() : id(-1), n_local(0), n_total(0), start_idx(-1),
   end_idx(-1), loc_map(nullptr), em_count(0), async_waits(nullptr),
-  refnum(nullptr), mismatches(nullptr), call_fn(nullptr), em_tab(nullptr), warp_ems(0), inline_ems(0) {}
+  refnum(nullptr), mismatches(nullptr), call_fn(nullptr), em_tab(nullptr), warp_ems(0), inline_ems(0),
+  em_cap(EM_CNT_MAX) {}
 
   __device__ bool warp_em(int ep) const { return ep >= 0 && ep < 64 && ((warp_ems >> ep) & 1ULL); }
 
@@ -117,7 +125,7 @@ struct chare_proxy_base {
   // Thread 0: runs inline entry method ep; the entry method that the block
   // runs next on the same chare and argument, or -1.
   __device__ int run_inline(int idx, int ep, void* arg) {
-    return reinterpret_cast<em_inline_fn>(em_tab[ep])(this, idx, arg);
+    return reinterpret_cast<em_inline_fn>(em_tab[INLINE_EM_MAX + 1 + ep])(this, idx, arg);
   }
 
   // Proxies come from the PE arena (shared memory when there is room), so
@@ -134,8 +142,8 @@ struct chare_proxy_base {
   // block). The scheduler decides the refnum match (refnum_matches, the
   // rule of include/chare.h:181-195) in one thread before it calls: the
   // entry method may change the chare's refnum at once, so the threads must
-  // not test it again here. Returns true (false, with BAD_TARGET, for an
-  // inline entry method).
+  // not test it again here. Returns true. An inline entry method is not run:
+  // BAD_TARGET.
   __device__ virtual bool call(int idx, int ep, void* arg, int ref) = 0;
   // Frees the local chares and tables (the runtime calls it when a run ends
   // and then deletes the proxy).
@@ -171,6 +179,8 @@ enum : int {
   ERR_NO_MEMORY = 17,
   ERR_TOO_MANY_WAITS = 19,
 };
+// Registers fn as the proxy's next entry method, an inline one.
+__device__ void add_inline_em(chare_proxy_base* proxy, em_inline_fn fn);
 // Registers proxy `id` in the scheduler's on-chip lookup cache.
 __device__ void cache_proxy(int id, chare_proxy_base* p);
 template <class T>
@@ -231,7 +241,7 @@ struct chare_proxy : chare_proxy_base {
   // Add entry method to table (single-threaded)
   template <void Func(C&, void*)>
   __device__ void add_entry_method() {
-    if (em_tab == nullptr || em_count >= EM_CNT_MAX) {
+    if (em_tab == nullptr || em_count >= em_cap) {
       detail::report_error(detail::ERR_TOO_MANY_EMS, id, em_count);
       return;
     }
@@ -272,20 +282,11 @@ struct chare_proxy : chare_proxy_base {
   }
   template <int Func(C&, void*)>
   __device__ void add_inline_entry_method() {
-    if (em_tab == nullptr || em_count >= 64) {
-      detail::report_error(detail::ERR_TOO_MANY_EMS, id, em_count);
-      return;
-    }
-    inline_ems |= 1ULL << em_count;
-    em_tab[em_count++] = reinterpret_cast<em_entry_fn>(&chare_proxy<C>::template em_inline_entry<Func>);
+    detail::add_inline_em(this, &chare_proxy<C>::template em_inline_entry<Func>);
   }
 
   __device__ static bool call_static(chare_proxy_base* base, int idx, int ep, void* arg) {
     chare_proxy<C>* self = static_cast<chare_proxy<C>*>(base);
-    if (self->inline_em(ep)) {  // the scheduler's thread 0 alone runs those
-      if (threadIdx.x == 0) detail::report_error(detail::ERR_BAD_TARGET, self->id, ep);
-      return false;
-    }
     self->em_tab[ep](base, idx, arg);
     return true;
   }
