@@ -382,6 +382,13 @@ namespace detail {
 void* pe_alloc(size_t) { return nullptr; }  // the device heap (new) serves every object here
 bool pe_owns(const void*) { return false; }
 chare_proxy_table& my_proxy_table() { return me_pe().table; }
+void add_inline_em(chare_proxy_base* p, em_inline_fn fn) {
+  const int ep = p->em_count++;
+  p->inline_ems |= 1ULL << ep;
+  p->em_cap = INLINE_EM_MAX;
+  p->em_tab[ep] = nullptr;  // the block never runs it
+  p->em_tab[INLINE_EM_MAX + 1 + ep] = reinterpret_cast<em_entry_fn>(fn);
+}
 void cache_proxy(int, chare_proxy_base*) {}
 void report_error(int code, int a, int b) { rt::set_error(code, a, b); }
 }  // namespace detail
