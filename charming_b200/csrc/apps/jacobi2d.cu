@@ -49,7 +49,7 @@ struct japp {
   __device__ static int pipeline() { return (int)g_app.a[3]; }
   __device__ static int tile_w() { return (int)g_app.a[4]; }
   __device__ static int halo_mode() { return (int)g_app.a[5]; }
-  // multi-sweep passes: 0 phase-split items, 1 the single-loop items
+  // multi-sweep passes: 0 steady steps without boundary tests, 1 every step with them
   __device__ static bool deep_lean() { return g_app.a[9] == 0; }
   __device__ static const jac::chare_desc* chares() {
     return reinterpret_cast<const jac::chare_desc*>(g_app.p[0]);
@@ -308,13 +308,7 @@ __device__ void count_nbrs(JBlock& c, const jac::chare_desc& d) {
   c.nbx = nx;
 }
 
-// Packs the boundary regions of buf[cur] for every neighbour straight into
-// their inbox rings (zero-copy) and publishes them together: the ring
-// reservations, the packing loads and the publishing fences of the messages
-// overlap (refnum = pass in halo_mode 1). phase 0: every neighbour (the
-// one-phase exchange); 1: left and right; 2: top and bottom, with the ghost
-// columns the left/right halos of this pass filled. All threads.
-// The halos of one batch: one copy per block, written by thread 0 (a
+// The packed halos of one batch: one copy per block, written by thread 0 (a
 // private copy in every thread was local memory, about 350 bytes per thread
 // per batch).
 struct halo_batch {
@@ -460,6 +454,12 @@ __device__ void put_halos(JBlock& c, const jac::chare_desc& d, int phase) {
   if (threadIdx.x == 0) add_pe_cyc(1, pe_clock() - t0);
 }
 
+// Packs the boundary regions of buf[cur] for every neighbour straight into
+// their inbox rings (zero-copy) and publishes them together: the ring
+// reservations, the packing loads and the publishing fences of the messages
+// overlap (refnum = pass in halo_mode 1). phase 0: every neighbour (the
+// one-phase exchange); 1: left and right; 2: top and bottom, with the ghost
+// columns the left/right halos of this pass filled. All threads.
 // Out of line, like the other paths that a chare with the default options
 // does not take (and the sweeps): inlined into the entry methods, their
 // registers were saved and restored by every thread on every delivery.

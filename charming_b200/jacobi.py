@@ -2,8 +2,10 @@
 
 Mirrors the reference's Jacobi example program (examples/jacobi2d/
 jacobi2d.cu): a Dirichlet problem is decomposed into a px x py chare array,
-chares exchange halos as messages every sweep, and the sweep is the
-5-point average (c + l + r + u + d) * 0.2.  Grids are (ny+2) x (nx+2)
+chares exchange halos (every `depth` sweeps: the boundary values are written
+into the neighbours' ghost zones and a message to each says so; with
+halo_mode 1, corner messages or the bulk-copy sweep they travel inside the
+messages), and the sweep is the 5-point average (c + l + r + u + d) * 0.2.  Grids are (ny+2) x (nx+2)
 row-major arrays whose outer ring is the fixed boundary.
 """
 from __future__ import annotations

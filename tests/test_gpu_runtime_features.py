@@ -142,11 +142,11 @@ def test_gpu_level_decomp1d_matches_oracle():
 
 @pytest.mark.parametrize("nx,ny,nz,sweeps,seed", [
     (6, 5, 4, 1, 1), (17, 9, 11, 3, 2), (33, 7, 13, 5, 3),   # the golden fixtures' shapes
-    (64, 48, 40, 4, 5),                                     # whole tiles
-    (97, 35, 70, 7, 6),                                     # ragged tiles, several z runs
-    # even row pitch: the TMA plane-ring kernel
-    (32, 16, 9, 4, 9),                                      # exactly one box
-    (94, 35, 70, 3, 7),                                     # ragged tiles, several z runs
+    (64, 48, 40, 4, 5),                                     # two strips, even rows
+    (97, 35, 70, 7, 6),                                     # ragged strips, several z runs
+    # even rows (no row copies)
+    (32, 16, 9, 4, 9),                                      # a row of 17 vectors: the narrowest in strips
+    (94, 35, 70, 3, 7),                                     # ragged strips, several z runs
     (62, 16, 300, 2, 8),                                    # long z runs, more planes than slots
 ])
 def test_jacobi3d_matches_oracle(rt, nx, ny, nz, sweeps, seed):
