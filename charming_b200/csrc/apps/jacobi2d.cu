@@ -147,7 +147,8 @@ __shared__ charm::chare_proxy<JBlock>* jproxy;
 // kept on chip and stored through to japp::pe_ns() after every update (a
 // store only: no read of global memory on the message path).
 // Slots: 0 sweeps, 1 halo sends (all of send_halos), 2 halo entry methods
-// (with halos put into the ghost zones: their notes),
+// (with halos put into the ghost zones: the inline ones, which take their
+// notes and the residual tree's messages),
 // 3 of the sends: up to the ring space taken, 4 of the sends: publishing,
 // 5 of the sends: up to the reservation call.
 constexpr int PE_NS_SLOTS = 8;
@@ -160,11 +161,14 @@ __device__ __forceinline__ void add_pe_cyc(int k, unsigned long long cyc) {
   s_pe_ns[k] += cyc;
   japp::pe_ns()[PE_NS_SLOTS * blockIdx.x + k] = s_pe_ns[k];
 }
-// Notes only add to their timer; the sweep that follows the last ones of a
-// pass stores it.
-__device__ __forceinline__ void add_sweep_cyc(unsigned long long cyc) {
+// With halos put into the ghost zones, timer 2 is the scheduler's own of the
+// inline entry methods, stored after each sweep (a timer in the notes' entry
+// method cost a 512^2 solve 0.7 %).
+__device__ __forceinline__ void add_sweep_cyc(bool puts, unsigned long long cyc) {
   add_pe_cyc(0, cyc);
-  japp::pe_ns()[PE_NS_SLOTS * blockIdx.x + 2] = s_pe_ns[2];
+#if !defined(CHARMING_HOST_EMULATION) || defined(EMU_RT)
+  if (puts) japp::pe_ns()[PE_NS_SLOTS * blockIdx.x + 2] = charm::rt::pes()->stats[charm::rt::ST_INLINE_CYC];
+#endif
 }
 __shared__ charm::chare_proxy<JServer>* sproxy;
 
@@ -203,6 +207,14 @@ __device__ __noinline__ bool sweep_pipeline(const jac::chare_desc& d, jac::block
 }
 #endif
 
+// Halos go straight into the neighbours' ghost zones, with a note each. A
+// note's sender is at most one pass ahead of its receiver, so what it writes
+// (the ghost zone of buffer pass & 1) is neither read nor written by the pass
+// that the receiver may still be running.
+__device__ __forceinline__ bool puts_halos(const jac::chare_desc& d) {
+  return japp::halo_mode() == 0 && !japp::pipeline() && (d.depth == 1 || d.ext > 0);
+}
+
 // One pass of L sweeps buf[cur] -> buf[cur^1]; returns the block's residual
 // sum of the pass's first sweep (FP64, deterministic) when resid is set.
 // All threads.
@@ -236,7 +248,7 @@ __device__ double sweep_block(const jac::chare_desc& d, int cur, bool resid, int
                 : jac::sweep_direct<T, false>(in, out, d.w, d.h);
     __syncthreads();
   }
-  if (threadIdx.x == 0) add_sweep_cyc(pe_clock() - t0);
+  if (threadIdx.x == 0) add_sweep_cyc(puts_halos(d), pe_clock() - t0);
   return resid ? suite::block_sum_f64(acc) : 0.0;
 }
 
@@ -319,14 +331,6 @@ struct halo_batch {
   int n;
 };
 __shared__ halo_batch s_halos;
-
-// Halos go straight into the neighbours' ghost zones, with a note each. A
-// note's sender is at most one pass ahead of its receiver, so what it writes
-// (the ghost zone of buffer pass & 1) is neither read nor written by the pass
-// that the receiver may still be running.
-__device__ __forceinline__ bool puts_halos(const jac::chare_desc& d) {
-  return japp::halo_mode() == 0 && !japp::pipeline() && (d.depth == 1 || d.ext > 0);
-}
 
 // The puts of one batch, like halo_batch: rectangles of nr rows of nu units
 // (16-byte vectors, or single elements where a row of either side does not

@@ -245,7 +245,7 @@ __device__ __forceinline__ int stale(const JBlock& c, unsigned gen, int fresh_ep
 
 // A neighbour's halo of hh->pass lies in the ghost zone: count it; the block
 // runs when the chare can go on (the conditions of pump()).
-__device__ __forceinline__ int count_note(JBlock& c, void* arg) {
+__device__ int in_note(JBlock& c, void* arg) {
   const jac::halo_hdr* hh = reinterpret_cast<const jac::halo_hdr*>(arg);
   const int dir = hh->dir, pass = hh->pass;
   if (const int s = stale(c, hh->gen, EP_FRESH_NOTE)) return s;
@@ -258,12 +258,6 @@ __device__ __forceinline__ int count_note(JBlock& c, void* arg) {
   if (!c.started || c.waiting || c.sent < c.pass) return -1;  // (the start pumps; so does a decision)
   if (c.desc.ext > 0 && c.sent_y < c.pass) return c.gotx[c.pass & 1] == c.nbx ? EP_PUMP : -1;
   return c.got[c.pass & 1] == c.nbr_count ? EP_PUMP : -1;
-}
-__device__ int in_note(JBlock& c, void* arg) {
-  const unsigned long long t0 = pe_clock();
-  const int next = count_note(c, arg);
-  s_pe_ns[2] += pe_clock() - t0;
-  return next;
 }
 
 __device__ int in_partial(JBlock& c, void* arg) {

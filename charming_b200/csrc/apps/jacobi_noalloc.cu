@@ -85,8 +85,10 @@ int scratch_on_current_device(void** out, int* sms) {
 constexpr int NA_U = 4;
 
 // v: the lane's vector, own: it stores it; rows r0 .. r1 - 1 (none if r1 <= r0)
-// in `run` + 2 L steps, the same number for all lanes of the warp.
-template <typename T, int L, bool ALIGNED, bool FIX>
+// in `run` + 2 L steps, the same number for all lanes of the warp. GRP: items of
+// fewer lanes than a warp's, compiled apart (one kernel for both made wide grids
+// 1 to 2 % slower).
+template <typename T, int L, bool ALIGNED, bool FIX, bool GRP>
 __device__ __forceinline__ void noalloc_item(const T* __restrict__ src, T* __restrict__ dst, int nx, int ny,
     int v, bool own, int r0, int r1, int run) {
   constexpr int V = jac::traits<T>::VEC, LH = (L + 1) / 2, U = NA_U;
@@ -103,7 +105,7 @@ __device__ __forceinline__ void noalloc_item(const T* __restrict__ src, T* __res
   }
   ln.fix_r0 = 0;
   ln.fix_r1 = ny + 1;
-  const int qs = r0 - L, qe = r1 - 1 + L, qend = r0 + run - 1 + L;
+  const int qs = r0 - L, qe = r1 - 1 + L, qend = GRP ? r0 + run - 1 + L : qe;
   // columns and rows off the grid: its nearest ones, never used by a result
   int off[V];
 #pragma unroll
@@ -169,24 +171,24 @@ __device__ __forceinline__ void noalloc_item(const T* __restrict__ src, T* __res
   }
 }
 
-template <typename T, int L, bool ALIGNED>
+template <typename T, int L, bool ALIGNED, bool GRP>
 __global__ void __launch_bounds__(128) noalloc_pass_kernel(const T* __restrict__ src, T* __restrict__ dst, int nx,
     int ny, int strips, int group, int run_rows, int warps) {
   constexpr int V = jac::traits<T>::VEC, E = (L + V - 1) / V, SS = 32 - 2 * E;
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = (int)(threadIdx.x & 31);
   if (w >= warps) return;
   const int nv = (nx + 2 + V - 1) / V;
-  if (group < 32) {
+  if (GRP) {
     const int v = lane & (group - 1), r0 = (w * (32 / group) + lane / group) * run_rows;
-    noalloc_item<T, L, ALIGNED, true>(src, dst, nx, ny, v, v < nv, r0, min(ny + 2, r0 + run_rows), run_rows);
-    return;
+    noalloc_item<T, L, ALIGNED, true, true>(src, dst, nx, ny, v, v < nv, r0, min(ny + 2, r0 + run_rows), run_rows);
+  } else {
+    const int own0 = w % strips * SS, nown = min(SS, nv - own0), v = own0 - E + lane;
+    const bool own = lane >= E && lane < E + nown;
+    const int r0 = w / strips * run_rows, r1 = min(ny + 2, r0 + run_rows);
+    const bool edge = own0 - E <= 0 || (own0 + nown + E) * V > nx + 1 || r0 - L <= 0 || r1 - 1 + L >= ny + 1;
+    if (edge) noalloc_item<T, L, ALIGNED, true, false>(src, dst, nx, ny, v, own, r0, r1, 0);
+    else noalloc_item<T, L, ALIGNED, false, false>(src, dst, nx, ny, v, own, r0, r1, 0);
   }
-  const int own0 = w % strips * SS, nown = min(SS, nv - own0), v = own0 - E + lane;
-  const bool own = lane >= E && lane < E + nown;
-  const int r0 = w / strips * run_rows, r1 = min(ny + 2, r0 + run_rows);
-  const bool edge = own0 - E <= 0 || (own0 + nown + E) * V > nx + 1 || r0 - L <= 0 || r1 - 1 + L >= ny + 1;
-  if (edge) noalloc_item<T, L, ALIGNED, true>(src, dst, nx, ny, v, own, r0, r1, r1 - r0);
-  else noalloc_item<T, L, ALIGNED, false>(src, dst, nx, ny, v, own, r0, r1, r1 - r0);
 }
 
 constexpr int NA_LMAX = 8;
@@ -226,7 +228,8 @@ void launch_pass(const T* src, T* dst, int nx, int ny, const pass_plan& p, bool 
   // few warps: blocks of one warp, so that they spread over the SMs
   const int threads = p.warps <= 4 * sms ? 32 : p.warps <= 8 * sms ? 64 : 128;
   const int blocks = (int)(((long long)p.warps * 32 + threads - 1) / threads);
-  auto fn = aligned ? noalloc_pass_kernel<T, L, true> : noalloc_pass_kernel<T, L, false>;
+  auto fn = p.group < 32 ? (aligned ? noalloc_pass_kernel<T, L, true, true> : noalloc_pass_kernel<T, L, false, true>)
+                         : (aligned ? noalloc_pass_kernel<T, L, true, false> : noalloc_pass_kernel<T, L, false, false>);
   fn<<<blocks, threads, 0, 0>>>(src, dst, nx, ny, p.strips, p.group, p.run_rows, p.warps);
 }
 template <typename T>

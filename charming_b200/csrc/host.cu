@@ -244,7 +244,10 @@ int collect_run(double kernel_ms) {
   for (int p = 0; p < n_local; p++) idle += (double)st[(size_t)p * N_STATS + ST_IDLE_CYC];
   s.idle_ms = (n_local && g.prop.clockRate > 0) ? idle / n_local / (double)g.prop.clockRate : 0.0;
   double em = 0;
-  for (int p = 0; p < n_local; p++) em += (double)st[(size_t)p * N_STATS + ST_EM_CYC];
+  for (int p = 0; p < n_local; p++) {
+    const unsigned long long* q = &st[(size_t)p * N_STATS];
+    em += (double)(q[ST_EM_CYC] + q[ST_INLINE_CYC]);
+  }
   s.em_ms = (n_local && g.prop.clockRate > 0) ? em / n_local / (double)g.prop.clockRate : 0.0;
   double tk = 0, sp = 0;
   for (int p = 0; p < n_local; p++) {

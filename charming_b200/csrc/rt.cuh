@@ -104,12 +104,13 @@ enum : int {
   ST_SPACE_WAITS,     // sends that waited for ring space
   ST_LOOP_NS,         // ns spent in the scheduler loop
   ST_IDLE_CYC,        // SM cycles spent waiting on an empty inbox
-  ST_EM_CYC,          // SM cycles spent inside entry methods
+  ST_EM_CYC,          // SM cycles spent inside entry methods that the block or a warp runs
   ST_DEFERRED,        // sends moved to the outbox (destination ring full)
   ST_TICKET_NS,       // ns the reserving thread waited for its ticket atomics
   ST_SPACE_NS,        // ns it then waited for ring space (head cache and waits)
   ST_BATCHED,         // deliveries run beside others in a batch of warp-level entry methods
-  N_STATS = 14
+  ST_INLINE_CYC,      // SM cycles spent inside inline entry methods
+  N_STATS = 15
 };
 
 constexpr int MAX_DEVS = 8;  // GPUs of one NVSwitch domain

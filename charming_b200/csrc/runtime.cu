@@ -1408,7 +1408,7 @@ __device__ bool inline_done(pe_state* ps, chare_proxy_base* p, int idx, int* ep,
   if (!p->inline_em(*ep)) return false;
   const long long c0 = clock64();
   const int next = p->run_inline(idx, *ep, arg);
-  ps->stats[ST_EM_CYC] += (unsigned long long)(clock64() - c0);
+  ps->stats[ST_INLINE_CYC] += (unsigned long long)(clock64() - c0);
   if (next < 0) {
     if ((++ps->stats[ST_DELIVERED] & 15) == 0) stamp_progress(ps->my_pe);
     return true;

@@ -244,7 +244,8 @@ typedef struct charming_jacobi_info {
   double sweep_ms_mean;       /* last run: mean over busy PEs              */
   double send_ms_mean;        /* last run: mean time packing/sending halos */
   double halo_ms_mean;        /* last run: mean time in halo entry methods (default halo
-                               * mode: counting the notes of the halos put) */
+                               * mode: in inline ones, which take the notes of the
+                               * halos put and the residual messages) */
   /* the next three: builds with -DCHARMING_PROFILE only (else 0) */
   double send_reserve_ms_mean;  /* of send_ms_mean: taking the ring space    */
   double send_publish_ms_mean;  /* of send_ms_mean: publishing the messages  */
