@@ -164,10 +164,9 @@ __device__ __forceinline__ void add_pe_cyc(int k, unsigned long long cyc) {
 // With halos put into the ghost zones, timer 2 is the scheduler's own of the
 // inline entry methods, stored after each sweep (a timer in the notes' entry
 // method cost a 512^2 solve 0.7 %).
-__device__ __forceinline__ void add_sweep_cyc(bool puts, unsigned long long cyc) {
-  add_pe_cyc(0, cyc);
+__device__ __forceinline__ void store_inline_cyc() {
 #if !defined(CHARMING_HOST_EMULATION) || defined(EMU_RT)
-  if (puts) japp::pe_ns()[PE_NS_SLOTS * blockIdx.x + 2] = charm::rt::pes()->stats[charm::rt::ST_INLINE_CYC];
+  japp::pe_ns()[PE_NS_SLOTS * blockIdx.x + 2] = charm::rt::pes()->stats[charm::rt::ST_INLINE_CYC];
 #endif
 }
 __shared__ charm::chare_proxy<JServer>* sproxy;
@@ -248,7 +247,7 @@ __device__ double sweep_block(const jac::chare_desc& d, int cur, bool resid, int
                 : jac::sweep_direct<T, false>(in, out, d.w, d.h);
     __syncthreads();
   }
-  if (threadIdx.x == 0) add_sweep_cyc(puts_halos(d), pe_clock() - t0);
+  if (threadIdx.x == 0) add_pe_cyc(0, pe_clock() - t0);
   return resid ? suite::block_sum_f64(acc) : 0.0;
 }
 
