@@ -624,7 +624,7 @@ struct deep_stream {
 // keeps need few register moves. sweep alone, 148 blocks of 2048 x 221, FP64, 6 levels:
 // 272 us per pass (1480 GLUP/s), 327 with the whole window kept and a branch
 // per level; FP32 155 us (199); 128 x 128 FP64 25.8 us (31.9). The FP64
-// pipe is 55 % busy, the shuffles' pipe 58 %, the issue slots 74 %.
+// pipe is 53 % busy, the shuffles' wavefronts 62 %, the issue slots 69 %.
 template <typename T, bool RESID, int L, int P>
 __device__ __forceinline__ double deep_item(const block_view<T>& in, const block_view<T>& out, int w,
     const deep_lane<T>& ln, int r0, int r1, int lane, typename vec_of<T>::type* ring, bool lean) {
