@@ -162,8 +162,9 @@ __device__ __forceinline__ void add_pe_cyc(int k, unsigned long long cyc) {
   japp::pe_ns()[PE_NS_SLOTS * blockIdx.x + k] = s_pe_ns[k];
 }
 // With halos put into the ghost zones, timer 2 is the scheduler's own of the
-// inline entry methods, stored after each sweep (a timer in the notes' entry
-// method cost a 512^2 solve 0.7 %).
+// inline entry methods, stored when a chare finishes (a timer in the notes'
+// entry method cost a 512^2 solve 0.7 %, a store after every sweep, which the
+// next release waits for, 3 % at one sweep per exchange).
 __device__ __forceinline__ void store_inline_cyc() {
 #if !defined(CHARMING_HOST_EMULATION) || defined(EMU_RT)
   japp::pe_ns()[PE_NS_SLOTS * blockIdx.x + 2] = charm::rt::pes()->stats[charm::rt::ST_INLINE_CYC];
@@ -564,6 +565,7 @@ __device__ void finish(JBlock& c, const jac::chare_desc& d) {
     s_last = 0;
   } else if (threadIdx.x == 0) {
     c.done = 1;
+    if (puts_halos(d)) store_inline_cyc();
     japp::final_buf()[c.i] = c.cur;
     const jac::prob_desc& p = c.prob;
     if (p.root == c.i) {

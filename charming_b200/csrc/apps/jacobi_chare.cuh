@@ -87,7 +87,6 @@ __device__ void advance(JBlock& c, const jac::chare_desc& d) {
     c.cur ^= 1;
     c.pass++;
     c.iter += L;
-    if (puts_halos(d)) store_inline_cyc();
     if (resid) {
       c.own = part;
       c.have_own = 1;
